@@ -96,10 +96,12 @@ typedef struct {
   int arith;                    /* pm_arith (FP64 sweeps) */
   int write_log;                /* 1: append the reference log rows to log_file_name */
   int mixed_inner;              /* FP32 sweeps per FP64 correction (0 = it_eval) */
-  int kernel;                   /* correction sweep of the mixed form: -1 autotune
-                                   (default: time the kernels 10, 9, 8, 6, 5, 7, 2 on
-                                   the problem; the first is kept unless another is
-                                   at least 5 % faster),
+  int kernel;                   /* correction sweep of the mixed form: -1 automatic
+                                   (default: 13, its block size timed on the
+                                   problem; for media whose offsets its records do
+                                   not hold, kernels 10, 9, 8, 6, 5, 7, 2 are timed
+                                   and the first is kept unless another is at least
+                                   5 % faster),
                                    0 TMA z-march 32x16 tiles, 3 TMA
                                    z-march 32x8 tiles, 1 fluid-list gather, 2 fluid-list
                                    gather at four blocks per SM, 4 TMA bricks (one
@@ -113,10 +115,11 @@ typedef struct {
                                    positions prefetched, five blocks per SM without,
                                    11 / 12 the same with each chunk's positions
                                    staged in shared memory by bulk copies at five /
-                                   four blocks per SM, 13 the same with the six
-                                   positions and the metadata in one 16-byte packed
-                                   record per voxel (16-bit offsets) at five blocks
-                                   per SM */
+                                   four blocks per SM, 13 persistent sweep with the
+                                   six positions and the metadata in one 16-byte
+                                   packed record per voxel, the next record
+                                   prefetched, each sweep's launch overlapping the
+                                   one before */
   int brick[3];                 /* fluid-list order when kernel >= 0: brick extents
                                    x y z (voxels), 0 0 0 = lexicographic; kernel 4 takes
                                    32 8 8 (default), 32 8 4 or 32 4 4 */

@@ -174,9 +174,12 @@ pm_status device_sync(pm_problem* pr, const char* where) {
 
 // The FP32 correction sweep e_out = L(e_in) + r of the mixed form.
 pm_status correction_sweep(pm_problem* pr, int src) {
-  if (pr->kern == 13) {
-    CK(launch_dc_inner_cr(pr->Ec[src], pr->Ec[1 - src], pr->Rc, pr->crec, pr->cslot4,
-                          pr->cslot2, pr->nlist, pr->solver, pr->st));
+  if (pr->kern == 13 && pr->crec) {
+    CK(launch_dc_inner_cr(pr->Ec[src], pr->Ec[1 - src], pr->Rc, pr->crec, pr->cslot2, pr->nlist,
+                          pr->solver, pr->cvar, pr->st));
+  } else if (pr->kern == 13) {  // a medium whose offsets no record holds
+    CK(launch_dc_inner_c(pr->Ec[src], pr->Ec[1 - src], pr->Rc, pr->cmeta, pr->cslot4,
+                         pr->cslot2, pr->nlist, pr->solver, 5, pr->st));
   } else if (pr->kern == 11 || pr->kern == 12) {
     CK(launch_dc_inner_cb(pr->Ec[src], pr->Ec[1 - src], pr->Rc, pr->cmeta, pr->cslot4,
                           pr->cslot2, pr->nlist, pr->solver, pr->kern == 11 ? 5 : 4, pr->cerr,
@@ -273,10 +276,12 @@ pm_status choose_fp64_shapes(pm_problem* pr) {
 // (pm_compact.cu: fluid voxels only, six precomputed neighbour positions per
 // voxel; 3 / 4 CTAs per SM with the next positions prefetched, 5 without),
 // 11 and 12 the same sweep with each chunk's positions staged in shared
-// memory by bulk copies (5 / 4 CTAs per SM).
-// kernel < 0 times the fluid-list candidates on this problem (a few launches
-// each; the correction buffers are scratch until the first residual sweep)
-// and keeps the fastest.
+// memory by bulk copies (5 / 4 CTAs per SM), 13 the sweep over packed records
+// of the compact store (16 bytes of index data per voxel instead of 28).
+// kernel < 0 takes 13 and times its launch variants on this problem (a few
+// launches each; the correction buffers are scratch until the first residual
+// sweep); where the records cannot hold a medium's offsets it times the other
+// list kernels and keeps the fastest.
 pm_status zero_corrections(pm_problem* pr) {
   if (pr->E[0]) {
     CK(launch_zero4(pr->E[0], pr->g, pr->st));
@@ -295,9 +300,9 @@ void release_unused_store(pm_problem* pr) {
     pr->E[0] = pr->E[1] = pr->R = nullptr;
   } else {
     cudaFree(pr->carena);
-    cudaFree(pr->crec);
+    cudaFree(pr->crec_own);
     pr->carena = nullptr;
-    pr->crec = nullptr;
+    pr->crec = pr->crec_own = nullptr;
     pr->compact_ready = false;
     pr->cerr = nullptr;
     pr->c_base = pr->Ec[0] = pr->Ec[1] = pr->Rc = nullptr;
@@ -316,6 +321,7 @@ void release_unused_store(pm_problem* pr) {
 // serialised instead of timing each other's noise.
 struct Cand {
   int k, b[3];
+  int var = 0;  // kernel 13: launch variant (launch_dc_inner_cr)
 };
 using TuneKey = std::array<long long, 6>;
 std::mutex g_tune_mu;
@@ -326,10 +332,12 @@ TuneKey tune_key(const pm_problem* pr) {
           (long long)llround(20.0 * (double)pr->nlist / (double)pr->g.nvox)};
 }
 
-// The kernel a problem will use if it is already known (pinned, or tuned for
-// a problem alike), else -1: problem creation then allocates only its store.
+// The kernel a problem will use if it is already known (pinned, the packed
+// records, or tuned for a problem alike), else -1: problem creation then
+// allocates only its store.
 int known_kernel(const pm_problem* pr, int kernel) {
   if (kernel >= 0) return kernel;
+  if (compact_records_fit(pr->g, pr->nlist)) return 13;
   std::lock_guard<std::mutex> lock(g_tune_mu);
   auto hit = g_tuned.find(tune_key(pr));
   return hit != g_tuned.end() ? hit->second.k : -1;
@@ -356,8 +364,15 @@ pm_status choose_correction_kernel(pm_problem* pr, int kernel) {
     }
     if (cpt && !pr->compact_ready) {
       CK(compact_setup(pr->codes, pr->g, pr->list, pr->nlist, pr->cwords, pr->cslot4,
-                       pr->cslot2, pr->cmeta, pr->st, pr->crec));
+                       pr->cslot2, pr->cmeta, pr->st));
       pr->compact_ready = true;
+    }
+    if (k == 13 && !pr->crec && compact_records_fit(pr->g, pr->nlist)) {
+      // pinned: records of their own (the footprint counts them); else they
+      // take the place of the slots
+      pr->crec = pr->crec_own ? pr->crec_own : (uint4*)pr->cslot4;
+      CK(compact_records(pr->cmeta, pr->cslot4, pr->cslot2, pr->nlist, pr->crec, pr->cslot2,
+                         pr->st));
     }
     if (k == 0 || k == 3)
       CK(zmarch_create(&pr->zp, pr->g, pr->E[0], pr->E[1], pr->R, pr->codes, 0, k == 3));
@@ -381,27 +396,33 @@ pm_status choose_correction_kernel(pm_problem* pr, int kernel) {
   if (hit != g_tuned.end()) {
     pm_status s = make(hit->second.k, hit->second.b);
     if (s != PM_OK) return s;
+    pr->cvar = hit->second.var;
     release_unused_store(pr);
     return device_sync(pr, "kernel choice");
   }
-  // The TMA kernels (0, 3, 4), the bulk-staged compact sweeps (11, 12) and
-  // the packed-record sweep (13) lose alone on every medium measured so far
-  // and are left to explicit choice; timing them would only lengthen the
-  // set-up of every problem.
-  const Cand cands[] = {{10, {0, 0, 0}}, {9, {0, 0, 0}}, {8, {0, 0, 0}}, {6, {0, 0, 0}},
-                        {6, {32, 8, 8}}, {5, {0, 0, 0}}, {7, {0, 0, 0}}, {2, {0, 0, 0}}};
-  const int nc = 8;
-  // Each candidate: the best of three timings of five sweeps.  The first
-  // candidate is kept unless another one is at least 5 % faster.  Timed alone
-  // the compact kernels 10, 9 and 8 come within 1 % of each other (10.4 us on
-  // the 128^3 sphere pack), but when problems share the device (the tensor's
-  // three rotations) more resident warps win: 2.75 / 2.86 / 3.08 ms per
-  // 100-sweep step.  So the candidates are ordered by resident warps and only
-  // a clear win alone displaces the first.
-  float t[nc];
+  // The packed records win on every medium measured (pm_compact.cu), so only
+  // their launch variants are timed.  Without them: the TMA kernels (0, 3, 4)
+  // and the bulk-staged compact sweeps (11, 12) lose on every medium and are
+  // left to explicit choice.
+  std::vector<Cand> cands;
+  if (compact_records_fit(pr->g, pr->nlist))
+    cands = {{13, {0, 0, 0}, 0}, {13, {0, 0, 0}, 1}, {13, {0, 0, 0}, 2}};
+  else
+    cands = {{10, {0, 0, 0}}, {9, {0, 0, 0}}, {8, {0, 0, 0}}, {6, {0, 0, 0}},
+             {6, {32, 8, 8}}, {5, {0, 0, 0}}, {7, {0, 0, 0}}, {2, {0, 0, 0}}};
+  const int nc = (int)cands.size();
+  // Each candidate: the best of three timings of five sweeps.  Among the list
+  // kernels the first is kept unless another one is at least 5 % faster: timed
+  // alone 10, 9 and 8 come within 1 % of each other (10.4 us on the 128^3
+  // sphere pack), but when problems share the device more resident warps win,
+  // and they are ordered by those.  The launch variants of the records hold the
+  // same warps: 2 % (512^3: 254 us with CTAs of 1024 threads, 267 with 256).
+  const float margin = cands[0].k == 13 ? 0.98f : 0.95f;
+  std::vector<float> t(nc);
   for (int i = 0; i < nc; ++i) {
     pm_status s;
     if ((s = make(cands[i].k, cands[i].b)) != PM_OK) return s;
+    pr->cvar = cands[i].var;
     for (int w = 0; w < 2; ++w)
       if ((s = correction_sweep(pr, 0)) != PM_OK) return s;
     t[i] = 1e30f;
@@ -419,10 +440,11 @@ pm_status choose_correction_kernel(pm_problem* pr, int kernel) {
   int bi = 0;
   for (int i = 1; i < nc; ++i)
     if (t[i] < t[bi]) bi = i;
-  if (t[bi] > 0.95f * t[0]) bi = 0;
+  if (t[bi] > margin * t[0]) bi = 0;
   g_tuned[key] = cands[bi];
   pm_status s = make(cands[bi].k, cands[bi].b);
   if (s != PM_OK) return s;
+  pr->cvar = cands[bi].var;
   if ((s = zero_corrections(pr)) != PM_OK) return s;
   if ((s = device_sync(pr, "kernel autotune")) != PM_OK) return s;
   release_unused_store(pr);
@@ -483,6 +505,14 @@ pm_status dc_flush(pm_problem* pr) {
 }  // namespace
 
 pm_status pm::problem_flush(pm_problem* pr) { return dc_flush(pr); }
+
+pm_status pm::problem_pack(pm_problem* pr) {
+  if (!pr->compact() || pr->crec || !compact_records_fit(pr->g, pr->nlist)) return PM_OK;
+  pr->crec = (uint4*)pr->cslot4;
+  pr->kern = 13;
+  CK(compact_records(pr->cmeta, pr->cslot4, pr->cslot2, pr->nlist, pr->crec, pr->cslot2, pr->st));
+  return PM_OK;
+}
 
 namespace {
 
@@ -925,8 +955,8 @@ pm_status pm::problem_create(const pm_params* p, const uint8_t* geom, int rot_ax
       pr->cmeta = (unsigned*)(a + o_m);
       pr->cerr = (int*)(a + o_err);
       pr->cwords = (uint2*)(a + o_w);
-      // kernel 13's packed records (pinned only)
-      if (kk == 13) CKF(dev_alloc((void**)&pr->crec, sizeof(uint4) * nl));
+      // kernel 13's packed records, when pinned
+      if (p->kernel == 13) CKF(dev_alloc((void**)&pr->crec_own, sizeof(uint4) * nl));
       CKF(cudaMemsetAsync(pr->c_base, 0, 3 * sizeof(float4) * nl, pr->st));
       CKF(cudaMemsetAsync(pr->cerr, 0, sizeof(int), pr->st));
       pr->Ec[0] = pr->c_base;
@@ -968,7 +998,7 @@ pm_status pm_problem_destroy(pm_problem* pr) {
   cudaFree(pr->arena);
   cudaFree(pr->f32_base);
   cudaFree(pr->carena);
-  cudaFree(pr->crec);
+  cudaFree(pr->crec_own);
   pinned_release(pr->hout);
   if (pr->ev0) cudaEventDestroy(pr->ev0);
   if (pr->ev1) cudaEventDestroy(pr->ev1);

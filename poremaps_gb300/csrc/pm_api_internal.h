@@ -98,7 +98,12 @@ struct pm_problem {
   unsigned* cmeta = nullptr;
   uint2* cwords = nullptr;
   int* cerr = nullptr;  // bulk-staged compact sweep (kernels 11, 12): a wait ran out
-  uint4* crec = nullptr;  // packed records of kernel 13 (own allocation, kernel 13 pinned only)
+  // packed records of kernel 13: where the slots were (the server and the
+  // autotuned form; the escaped positions' y table then lies where cslot2
+  // was), or an allocation of their own (kernel 13 pinned)
+  uint4* crec = nullptr;
+  uint4* crec_own = nullptr;
+  int cvar = 0;           // launch variant of kernel 13
   double* partials = nullptr;
   double* dout = nullptr;
   double* hout = nullptr;  // pinned (a 256-byte slot of the process-wide pool)
@@ -154,6 +159,9 @@ long long problem_nvox(const pm_problem* pr);
 cudaStream_t problem_stream(const pm_problem* pr);
 // calc_flow pieces shared with the server
 pm_status iterate_n(pm_problem* pr, int n);
+// packs the compact store's slots into records in their place (kernel 13),
+// where they hold the medium's offsets
+pm_status problem_pack(pm_problem* pr);
 // mixed form: fold the FP32 correction into the FP64 state (no-op otherwise)
 pm_status problem_flush(pm_problem* pr);
 pm_status reduce(pm_problem* pr, int full);

@@ -60,6 +60,22 @@ __global__ void k_batch_residual(const SampleDesc* d, const WorkItem* items, int
   });
 }
 
+// One voxel of a correction sweep: over the packed records, or the full slots
+// where they do not hold the sample's offsets.
+template <int S, bool COHERENT>
+__device__ __forceinline__ void batch_inner_voxel(const SampleDesc& sd, const float4* Ein,
+                                                  float4* Eout, int q) {
+  const int sv = S ? S : sd.solver;
+  if (sd.rec) {
+    const uint4 rc = ld_record(sd.rec + q);
+    if (sv == 3) inner_r_voxel<3, COHERENT>(Ein, Eout, sd.R, rc, sd.ya, q, sd.nlist);
+    else inner_r_voxel<2, COHERENT>(Ein, Eout, sd.R, rc, sd.ya, q, sd.nlist);
+  } else {
+    if (sv == 3) inner_c_voxel<3, COHERENT>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, q);
+    else inner_c_voxel<2, COHERENT>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, q);
+  }
+}
+
 // At most 64 registers (1024 resident threads per SM at any block size the
 // server tunes): measured faster here than three blocks of 256 threads at
 // ~80 registers (54.2k against 50.8k solves/h on 32 uneven samples).
@@ -70,10 +86,7 @@ __global__ void __launch_bounds__(512, 2)
     const int a = (sd.ecur0 + round - 1) & 1;
     const float4* Ein = a ? sd.E1 : sd.E0;
     float4* Eout = a ? sd.E0 : sd.E1;
-    const int sv = S ? S : sd.solver;
-    if (sv == 3) inner_c_voxel<3>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, q);
-    else if (sv == 2) inner_c_voxel<2>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, q);
-    else inner_c_voxel<1>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, q);
+    batch_inner_voxel<S, false>(sd, Ein, Eout, q);
   });
 }
 
@@ -182,13 +195,8 @@ __global__ void __launch_bounds__(256, 4)
     const int a = (sd.ecur0 + k - 1) & 1;
     const float4* Ein = a ? sd.E1 : sd.E0;
     float4* Eout = a ? sd.E0 : sd.E1;
-    const int sv = S ? S : sd.solver;
-    for (int q = threadIdx.x; q < w.count; q += blockDim.x) {
-      const int i = w.start + q;
-      if (sv == 3) inner_c_voxel<3, true>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, i);
-      else if (sv == 2) inner_c_voxel<2, true>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, i);
-      else inner_c_voxel<1, true>(Ein, Eout, sd.R, sd.meta, sd.sa, sd.sb, i);
-    }
+    for (int q = threadIdx.x; q < w.count; q += blockDim.x)
+      batch_inner_voxel<S, true>(sd, Ein, Eout, w.start + q);
     __syncthreads();  // every store of the item is issued before the release
     if (threadIdx.x == 0) {
       __threadfence();

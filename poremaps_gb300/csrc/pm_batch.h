@@ -15,6 +15,9 @@ struct SampleDesc {
   const unsigned* meta;   // compact store: cases, flags per list position
   const int4* sa;         // compact store: x L, x R, y L, y R neighbour positions
   const int2* sb;         // compact store: z L, z R neighbour positions
+  const uint4* rec;       // packed records (null: meta, sa, sb), with the y table
+  const int2* ya;         // of the escaped positions
+  int nlist;
   const int* list;
   int solver;
   int ecur0;  // correction buffer the residual writes (mixed form)

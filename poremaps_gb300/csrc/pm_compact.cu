@@ -1,5 +1,5 @@
 // Compact correction store of the mixed-precision form (correction-sweep
-// kernels 8 and 9, and the server's batched sweeps).
+// kernels 8 to 13; the server's batched sweeps use its records).
 //
 // The FP32 correction e and residual r hold one float4 (u, v, w, p) per
 // fluid voxel, at the voxel's position in the lexicographic fluid list,
@@ -277,43 +277,51 @@ __global__ void k_compact_slots(const uint8_t* codes, Grid g, int nw, const int*
   }
 }
 
-// Packed records (kernel 13) from the slots and metadata.
-__global__ void k_pack_records(const unsigned* __restrict__ meta, const int4* __restrict__ sa,
-                               const int2* __restrict__ sb, int nlist, uint4* __restrict__ rec) {
+// Packed records (kernel 13) from the slots and metadata, and the absolute y
+// positions the escaped ones read.  rec may take the place of sa, ya of sb:
+// each thread reads its entries before it writes them.
+__global__ void k_pack_records(const unsigned* meta, const int4* sa, const int2* sb, int nlist,
+                               uint4* rec, int2* ya) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nlist; q += gridDim.x * blockDim.x) {
-    const int4 a = sa[q];
-    const int2 b = sb[q];
-    unsigned d[6];
-    bool ok = pack16(a.x, q, nlist, d[0]) & pack16(a.y, q, nlist, d[1]) &
-              pack16(a.z, q, nlist, d[2]) & pack16(a.w, q, nlist, d[3]) &
-              pack16(b.x, q, nlist, d[4]) & pack16(b.y, q, nlist, d[5]);
-    rec[q] = ok ? make_uint4(meta[q], d[0] | d[1] << 16, d[2] | d[3] << 16, d[4] | d[5] << 16)
-                : make_uint4(meta[q] | kMetaEscape, 0u, 0u, 0u);
+    CompactSlots sl;
+    sl.a = sa[q];
+    sl.b = sb[q];
+    const unsigned m = meta[q];
+    const Neighbours n = neighbours_of(m, sl);
+    rec[q] = pack_record(m, n, q, nlist);
+    ya[q] = make_int2(n.y0, n.y1);
   }
 }
 
-// The correction sweep over packed records (kernel 13): one 128-bit load of
-// index data per position; an escaped position (a periodic face more than
-// 32767 positions away) reads its full slots.  Persistent, no prefetch.
-template <int SOLVER, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_dc_inner_cr(const float4* __restrict__ E,
-                                                          float4* __restrict__ E2,
-                                                          const float4* __restrict__ R,
-                                                          const uint4* __restrict__ rec,
-                                                          const int4* __restrict__ sa,
-                                                          const int2* __restrict__ sb,
-                                                          int nlist) {
+// The correction sweep over packed records (kernel 13).  Persistent, one wave
+// of 1024 threads per SM; each thread has its next record in flight while the
+// current voxel's eight values arrive.  Launched programmatically: a CTA lets
+// the next kernel's CTAs in when it starts on its last positions (earlier, they
+// would take the place of other streams' CTAs), and they load their first
+// records and wait for this kernel's end before they touch a value.
+// Bound: the medium's values once they exceed L2 (64 bytes per voxel of e, r,
+// records and e2 against 76 with slots and metadata), the L1's gathers within
+// it.  Against kernels 10 / 9 (28 bytes of slots and metadata per voxel, plain
+// launches), per iteration of a solve: 48x48x64 pore 2.3 us (2.8), 128^3 pack
+// 7.8 (9.3), 157x93x211 9.5 (11.8), 256^3 38.9 (43.3), 512^3 309 (342).  The
+// streaming hint on r and the records is worth 8 % at 128^3 and 17 % when the
+// tensor's three problems share L2; bricks of the list instead of rows made no
+// difference at any size.
+template <int SOLVER, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+    k_dc_inner_cr(const float4* E, float4* E2, const float4* R, const uint4* __restrict__ rec,
+                  const int2* __restrict__ ya, int nlist) {
   const int stride = gridDim.x * blockDim.x;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nlist; q += stride) {
-    const uint4 r = __ldg(rec + q);
-    CompactSlots sl;
-    if (r.x & kMetaEscape) {
-      sl.a = __ldg(sa + q);
-      sl.b = __ldg(sb + q);
-    } else {
-      decode_record(r, q, nlist, sl);
-    }
-    inner_c_compute<SOLVER>(E, E2, R, q, r.x & ~kMetaEscape, sl);
+  int q = blockIdx.x * blockDim.x + threadIdx.x;
+  uint4 rc = make_uint4(0u, 0u, 0u, 0u);
+  if (q < nlist) rc = ld_record(rec + q);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (; q < nlist; q += stride) {
+    const int qn = q + stride;
+    if (qn >= nlist) asm volatile("griddepcontrol.launch_dependents;");
+    const uint4 next = ld_record(rec + (qn < nlist ? qn : q));
+    inner_r_voxel<SOLVER>(E, E2, R, rc, ya, q, nlist);
+    rc = next;
   }
 }
 
@@ -331,8 +339,7 @@ long long compact_words(const Grid& g) {
 }
 
 cudaError_t compact_setup(const uint8_t* codes, const Grid& g, const int* list, int nlist,
-                          uint2* words, int4* sa, int2* sb, unsigned* meta, cudaStream_t st,
-                          uint4* rec) {
+                          uint2* words, int4* sa, int2* sb, unsigned* meta, cudaStream_t st) {
   const int nw = (g.nx + 31) / 32;
   const long long nwords = compact_words(g) - 1;
   const int sms = sm_count();
@@ -341,23 +348,57 @@ cudaError_t compact_setup(const uint8_t* codes, const Grid& g, const int* list, 
   k_compact_slots<<<grid_for(nlist, 256, 16 * sms), 256, 0, st>>>(codes, g, nw, list, nlist,
                                                                    words, sa, sb, meta);
   count_launches(2);
-  if (rec && nlist > 0) {
-    k_pack_records<<<grid_for(nlist, 256, 16 * sms), 256, 0, st>>>(meta, sa, sb, nlist, rec);
-    count_launches(1);
-  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_dc_inner_cr(const float4* e, float4* e2, const float4* r, const uint4* rec,
-                               const int4* sa, const int2* sb, int nlist, int solver,
-                               cudaStream_t st) {
+bool compact_records_fit(const Grid& g, int nlist) { return records_fit(g, nlist); }
+
+cudaError_t compact_records(const unsigned* meta, const int4* sa, const int2* sb, int nlist,
+                            uint4* rec, int2* ya, cudaStream_t st) {
   if (nlist < 1) return cudaSuccess;
-  const int blocks = grid_for(nlist, 256, 5 * sm_count());
-  if (solver == 1) k_dc_inner_cr<1, 5><<<blocks, 256, 0, st>>>(e, e2, r, rec, sa, sb, nlist);
-  else if (solver == 2) k_dc_inner_cr<2, 5><<<blocks, 256, 0, st>>>(e, e2, r, rec, sa, sb, nlist);
-  else k_dc_inner_cr<3, 5><<<blocks, 256, 0, st>>>(e, e2, r, rec, sa, sb, nlist);
+  k_pack_records<<<grid_for(nlist, 256, 16 * sm_count()), 256, 0, st>>>(meta, sa, sb, nlist, rec,
+                                                                        ya);
   count_launches(1);
   return cudaGetLastError();
+}
+
+// A launch whose CTAs may become resident before the stream's previous kernel
+// has ended (they wait for it themselves).
+template <typename... P, typename... A>
+static cudaError_t launch_overlapped(void (*kernel)(P...), int blocks, int threads,
+                                     cudaStream_t st, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
+template <int THREADS>
+static cudaError_t inner_cr_launch(const float4* e, float4* e2, const float4* r, const uint4* rec,
+                                   const int2* ya, int nlist, int solver, cudaStream_t st) {
+  const int blocks = grid_for(nlist, THREADS, 1024 / THREADS * sm_count());
+  count_launches(1);
+  if (solver == 2)
+    return launch_overlapped(k_dc_inner_cr<2, THREADS>, blocks, THREADS, st, e, e2, r, rec, ya,
+                             nlist);
+  return launch_overlapped(k_dc_inner_cr<3, THREADS>, blocks, THREADS, st, e, e2, r, rec, ya,
+                           nlist);
+}
+
+cudaError_t launch_dc_inner_cr(const float4* e, float4* e2, const float4* r, const uint4* rec,
+                               const int2* ya, int nlist, int solver, int variant,
+                               cudaStream_t st) {
+  if (nlist < 1) return cudaSuccess;
+  // (solver 1 has no mixed form)
+  if (variant == 1) return inner_cr_launch<512>(e, e2, r, rec, ya, nlist, solver, st);
+  if (variant == 2) return inner_cr_launch<1024>(e, e2, r, rec, ya, nlist, solver, st);
+  return inner_cr_launch<256>(e, e2, r, rec, ya, nlist, solver, st);
 }
 
 template <int MINB, bool PF>

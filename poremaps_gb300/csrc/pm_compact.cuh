@@ -70,32 +70,73 @@ __device__ __forceinline__ unsigned make_meta(int cx, int cy, int cz, bool zfirs
   return m;
 }
 
-// Packed record of a list position (kernel 13): the metadata word and the six
-// slots as signed 16-bit offsets from the position itself,
-//   {meta, xL | xR << 16, yL | yR << 16, zL | zR << 16},
-// with kZeroSlot16 for the zero slot.  A position whose slots do not all fit
-// (an offset beyond +-32767: a periodic face more than one plane of fluid
-// away, or planes of more than 32767 fluid voxels) has kMetaEscape set and
-// reads its full slots instead.  16 bytes per position instead of 28.
-constexpr unsigned kMetaEscape = 1u << 31;
-constexpr int kZeroSlot16 = -32768;
+// Packed record of a list position (kernel 13 and the server's sweeps): 16
+// bytes instead of the 28 of slots and metadata.  Per axis the positions of the
+// two points (F, S) its neighbourhood case uses, as offsets from the position
+// itself (a value of its own, in z the offset of the zero slot, where there is
+// none):
+//   case     1  2  3  4  5  6
+//   F        -  -  l  r  l  l
+//   S        -  r  -  rr ll r
+// x offsets take 14 bits each (a row's fluid voxels), y offsets 16, z offsets
+// 28 (the whole list: a periodic z face); bits 0-10 of the first word are the
+// cases and the plane flags of the metadata.  A position whose y offsets do
+// not fit (a periodic y face of a plane of more than 32,767 fluid voxels) has
+// kRecEscape set and its absolute y positions in a table of their own.
+constexpr unsigned kRecMeta = 0x7ffu;
+constexpr unsigned kRecEscape = 1u << 11;
+constexpr int kNoneX = -(1 << 13), kNoneY = -(1 << 15);
 
-__device__ __forceinline__ bool pack16(int slot, int q, int nlist, unsigned& out) {
-  const int d = slot == nlist ? kZeroSlot16 : slot - q;
-  if (slot != nlist && (d < -32767 || d > 32767)) return false;
-  out = (unsigned)d & 0xFFFFu;
-  return true;
+__host__ __device__ __forceinline__ bool records_fit(const Grid& g, long long nlist) {
+  return g.nx < (1 << 13) && nlist < (1LL << 27) - 1;
 }
 
-__device__ __forceinline__ int unpack16(unsigned w, int hi, int q, int nlist) {
-  const int d = hi ? ((int)w >> 16) : ((int)(w << 16) >> 16);
-  return d == kZeroSlot16 ? nlist : q + d;
+struct Neighbours {  // list positions of F, S per axis
+  int x0, x1, y0, y1, z0, z1;
+};
+
+// The points F, S from the slots L, R (see CompactSlots).
+__device__ __forceinline__ Neighbours neighbours_of(unsigned meta, const CompactSlots& sl) {
+  int s[6] = {sl.a.x, sl.a.y, sl.a.z, sl.a.w, sl.b.x, sl.b.y};
+  for (int ax = 0; ax < 3; ++ax)
+    if (((meta >> (3 * ax)) & 7u) == 4u) {  // (rr, r) -> (r, rr)
+      const int t = s[2 * ax];
+      s[2 * ax] = s[2 * ax + 1];
+      s[2 * ax + 1] = t;
+    }
+  return {s[0], s[1], s[2], s[3], s[4], s[5]};
 }
 
-__device__ __forceinline__ void decode_record(uint4 rec, int q, int nlist, CompactSlots& sl) {
-  sl.a = make_int4(unpack16(rec.y, 0, q, nlist), unpack16(rec.y, 1, q, nlist),
-                   unpack16(rec.z, 0, q, nlist), unpack16(rec.z, 1, q, nlist));
-  sl.b = make_int2(unpack16(rec.w, 0, q, nlist), unpack16(rec.w, 1, q, nlist));
+__device__ __forceinline__ uint4 pack_record(unsigned meta, const Neighbours& n, int q,
+                                             int nlist) {
+  const int x0 = n.x0 == nlist ? kNoneX : n.x0 - q, x1 = n.x1 == nlist ? kNoneX : n.x1 - q;
+  int y0 = n.y0 == nlist ? kNoneY : n.y0 - q, y1 = n.y1 == nlist ? kNoneY : n.y1 - q;
+  const int z0 = n.z0 - q, z1 = n.z1 - q;
+  auto fits = [&](int pos, int d) { return pos == nlist || (d > kNoneY && d <= 32767); };
+  unsigned m = meta & kRecMeta;
+  if (!fits(n.y0, y0) || !fits(n.y1, y1)) {
+    m |= kRecEscape;
+    y0 = y1 = 0;
+  }
+  uint4 r;
+  r.x = m | ((unsigned)(z1 >> 8) & 0xfffffu) << 12;
+  r.y = ((unsigned)x0 & 0x3fffu) | ((unsigned)x1 & 0x3fffu) << 14 | ((unsigned)z1 & 0xfu) << 28;
+  r.z = ((unsigned)y0 & 0xffffu) | (unsigned)y1 << 16;
+  r.w = (unsigned)z0 << 4 | (((unsigned)z1 >> 4) & 0xfu);
+  return r;
+}
+
+__device__ __forceinline__ Neighbours unpack_record(const uint4& r, int q, int nlist) {
+  const int x0 = (int)(r.y << 18) >> 18, x1 = (int)(r.y << 4) >> 18;
+  const int y0 = (int)(r.z << 16) >> 16, y1 = (int)r.z >> 16;
+  Neighbours n;
+  n.x0 = x0 == kNoneX ? nlist : q + x0;
+  n.x1 = x1 == kNoneX ? nlist : q + x1;
+  n.y0 = y0 == kNoneY ? nlist : q + y0;
+  n.y1 = y1 == kNoneY ? nlist : q + y1;
+  n.z0 = q + ((int)r.w >> 4);
+  n.z1 = q + ((int)(r.x & ~0xfffu) >> 4 | (int)((r.w & 0xfu) << 4) | (int)(r.y >> 28));
+  return n;
 }
 
 __device__ __forceinline__ int word_rank(uint2 w, int x) {
@@ -160,6 +201,144 @@ __device__ __forceinline__ void inner_c_compute(const float4* __restrict__ E,
   float un, vn, wn, pn;
   update_fast_cases<float, SOLVER>(s, cx, cy, cz, un, vn, wn, pn);
   E2[i] = make_float4(un + r.x, vn + r.y, wn + r.z, pn + r.w);
+}
+
+// ---- the sweep over packed records
+
+// One velocity component of update_fast<float>: f holds its off-centre sum.
+template <int SOLVER>
+__device__ __forceinline__ float velocity(float c, float f, float centre, float dp, bool zero) {
+  f = fmaf(centre, c, f);
+  if (SOLVER == 3) {
+    const float t = fmaf(float(kDt / kRe * kOmega), f, float(1.0 - kOmega) * c);
+    return fmaf(float(-kDt * kOmega), dp, t);
+  }
+  float t = fmaf(float(kDt / kRe), f, c);
+  t = fmaf(float(-kDt), dp, t);
+  return zero ? 0.f : t;
+}
+
+// Wall stencil a c + cF F + cS S of a case, and which neighbours F and S are.
+struct CaseTerms {
+  float a, cF, cS;
+  bool s;           // S is not a second neighbour
+  bool lf, rf, r4;  // left / right neighbour fluid; the right one is F
+};
+
+__device__ __forceinline__ CaseTerms case_terms(unsigned c) {
+  const bool le2 = c <= 2, le3 = c <= 3, le5 = c <= 5;
+  CaseTerms k;
+  k.a = c == 1 ? -8.f : (le3 ? float(-16.0 / 3.0) : (le5 ? -5.f : -2.f));
+  k.cF = le2 ? 0.f : (le3 ? float(8.0 / 3.0) : (le5 ? 2.f : 1.f));
+  k.cS = c == 2 ? float(8.0 / 3.0) : (le3 ? 0.f : (le5 ? -0.2f : 1.f));
+  k.s = c - 4u >= 2u;
+  k.lf = !le2 && c != 4;
+  k.rf = !(c & 1u);
+  k.r4 = c == 4;
+  return k;
+}
+
+// The update of update_fast<float> from the centre and the points F, S of each
+// axis, its terms in the same order (a missing point is a zero, as is its
+// term), so every kernel gives the same values (a zero may differ in sign).
+template <int SOLVER>
+__device__ __forceinline__ float4 update_records(unsigned meta, const float4& C, const float4& XF,
+                                                 const float4& XS, const float4& YF,
+                                                 const float4& YS, const float4& ZF,
+                                                 const float4& ZS, const float4& r) {
+  const CaseTerms kx = case_terms(meta & 7u), ky = case_terms((meta >> 3) & 7u),
+                  kz = case_terms((meta >> 6) & 7u);
+  const float pc = (meta & kMetaZLast) ? 0.f : C.w;
+  const float zfw = (meta & kMetaZFirst) ? 0.f : ZF.w;
+  auto along = [](const CaseTerms& k, float f, float s) { return f + (k.s ? s : 0.f); };
+  auto right = [](const CaseTerms& k, float f, float s) {
+    return k.rf ? (k.r4 ? f : s) : 0.f;
+  };
+  float f = along(kx, XF.x, XS.x);
+  f = fmaf(ky.cF, YF.x, f);
+  f = fmaf(ky.cS, YS.x, f);
+  f = fmaf(kz.cF, ZF.x, f);
+  f = fmaf(kz.cS, ZS.x, f);
+  const float un =
+      velocity<SOLVER>(C.x, f, -2.f + ky.a + kz.a, kx.lf ? pc - XF.w : 0.f, !kx.lf);
+  f = along(ky, YF.y, YS.y);
+  f = fmaf(kx.cF, XF.y, f);
+  f = fmaf(kx.cS, XS.y, f);
+  f = fmaf(kz.cF, ZF.y, f);
+  f = fmaf(kz.cS, ZS.y, f);
+  const float vn =
+      velocity<SOLVER>(C.y, f, -2.f + kx.a + kz.a, ky.lf ? pc - YF.w : 0.f, !ky.lf);
+  f = along(kz, ZF.z, ZS.z);
+  f = fmaf(kx.cF, XF.z, f);
+  f = fmaf(kx.cS, XS.z, f);
+  f = fmaf(ky.cF, YF.z, f);
+  f = fmaf(ky.cS, YS.z, f);
+  const float wn =
+      velocity<SOLVER>(C.z, f, -2.f + kx.a + ky.a, kz.lf ? pc - zfw : 0.f, !kz.lf);
+  const float div = ((right(kz, ZF.z, ZS.z) - wn) + (right(ky, YF.y, YS.y) - vn)) +
+                    (right(kx, XF.x, XS.x) - un);
+  const float pn = fmaf(float(-kC2 * kDt), div, pc);
+  return make_float4(un + r.x, vn + r.y, wn + r.z, pn + r.w);
+}
+
+// Loads of values an earlier launch wrote, possibly while this one was already
+// resident (programmatic launch): not the read-only path.  COHERENT: written in
+// this launch by other CTAs, so past L1.
+template <bool COHERENT>
+__device__ __forceinline__ float4 ld_value(const float4* p) {
+  float4 v;
+  if (COHERENT)
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+  else
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+  return v;
+}
+
+// Loads of what a sweep reads once (residuals, records): past L1, and the first
+// to leave L2, so that the correction, which the next sweep reads again, stays.
+__device__ __forceinline__ unsigned long long stream_policy() {
+  unsigned long long p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p), "l"(stream_policy()));
+  return v;
+}
+
+// (set up long before any sweep: the read-only path)
+__device__ __forceinline__ uint4 ld_record(const uint4* p) {
+  uint4 v;
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p), "l"(stream_policy()));
+  return v;
+}
+
+// e2 = L(e) + r at list position q, record rc.
+template <int SOLVER, bool COHERENT = false>
+__device__ __forceinline__ void inner_r_voxel(const float4* E, float4* E2, const float4* R,
+                                              const uint4& rc, const int2* ya, int q, int nlist) {
+  Neighbours n = unpack_record(rc, q, nlist);
+  if (rc.x & kRecEscape) {
+    const int2 y = __ldg(ya + q);
+    n.y0 = y.x;
+    n.y1 = y.y;
+  }
+  const float4 C = ld_value<COHERENT>(E + q);
+  const float4 XF = ld_value<COHERENT>(E + n.x0), XS = ld_value<COHERENT>(E + n.x1);
+  const float4 YF = ld_value<COHERENT>(E + n.y0), YS = ld_value<COHERENT>(E + n.y1);
+  const float4 ZF = ld_value<COHERENT>(E + n.z0), ZS = ld_value<COHERENT>(E + n.z1);
+  const float4 r = ld_stream(R + q);
+  E2[q] = update_records<SOLVER>(rc.x, C, XF, XS, YF, YS, ZF, ZS, r);
 }
 
 // One voxel of the batched kernels.

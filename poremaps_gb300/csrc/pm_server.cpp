@@ -233,7 +233,8 @@ pm_status admit(pm_server* s) {
       continue;
     }
     // iteration 0 on its own: afterwards every block ends on a check iteration
-    if ((st = iterate_n(pr, 1)) == PM_OK) st = problem_flush(pr);
+    if (p.precision == PM_PREC_MIXED) st = problem_pack(pr);
+    if (st == PM_OK && (st = iterate_n(pr, 1)) == PM_OK) st = problem_flush(pr);
     if (st == PM_OK && cudaStreamSynchronize(problem_stream(pr)) != cudaSuccess)
       st = cuda_error(cudaGetLastError(), "admission sweep");
     if (st != PM_OK) {
@@ -484,6 +485,9 @@ pm_status rebuild(pm_server* s) {
       d.meta = pr->cmeta;
       d.sa = pr->cslot4;
       d.sb = pr->cslot2;
+      d.rec = pr->crec;
+      d.ya = pr->cslot2;
+      d.nlist = pr->nlist;
       d.ecur0 = 0;
       d.xcur0 = 0;
     } else {
