@@ -24,10 +24,11 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
           "--expt-relaxed-constexpr"]
 
-# (source, extra flags).  pm_kernels.cu holds the exact-arithmetic kernels and
-# must not contract multiply-adds (bitwise parity with the reference CPU code).
+# (source, extra flags).  pm_kernels.cu and pm_wave.cu hold the exact-arithmetic
+# kernels and must not contract multiply-adds (bitwise parity with the reference CPU code).
 UNITS = [
     ("pm_kernels.cu", ["-fmad=false"]),
+    ("pm_wave.cu", ["-fmad=false"]),
     ("pm_fast.cu", []),
     ("pm_compact.cu", []),
     ("pm_zmarch.cu", []),

@@ -156,9 +156,10 @@ pm_status validate(const pm_params* p) {
 pm_status device_sync(pm_problem* pr, const char* where) {
   cudaError_t e = cudaStreamSynchronize(pr->st);
   if (e != cudaSuccess) return cuda_error(e, where);
-  int* flags[3] = {pr->zp ? zmarch_error_flag(pr->zp) : nullptr,
+  int* flags[4] = {pr->zp ? zmarch_error_flag(pr->zp) : nullptr,
                    pr->bp ? brick_error_flag(pr->bp) : nullptr,
-                   (pr->kern == 11 || pr->kern == 12) ? pr->cerr : nullptr};
+                   (pr->kern == 11 || pr->kern == 12) ? pr->cerr : nullptr,
+                   pr->werr};
   for (int* f : flags) {
     if (!f) continue;
     int flag = 0;
@@ -166,7 +167,7 @@ pm_status device_sync(pm_problem* pr, const char* where) {
     if (e != cudaSuccess) return cuda_error(e, where);
     if (flag) {
       cudaMemset(f, 0, sizeof(int));
-      return set_error(PM_ERR_CUDA, "%s: a TMA wait of the correction sweep timed out", where);
+      return set_error(PM_ERR_CUDA, "%s: a wait of the sweep timed out", where);
     }
   }
   return PM_OK;
@@ -451,44 +452,6 @@ pm_status choose_correction_kernel(pm_problem* pr, int kernel) {
   return PM_OK;
 }
 
-// Block size of the reference-order wavefront, timed on the problem: a few
-// iterations on the second state buffer (a copy of the initial state, restored
-// afterwards) per candidate; every shape gives bitwise identical fields.
-// Shared across alike problems as the correction-sweep choice is.
-pm_status choose_wavefront_shape(pm_problem* pr) {
-  static std::mutex mu;
-  static std::map<std::array<long long, 5>, int> tuned;
-  std::lock_guard<std::mutex> lock(mu);
-  const std::array<long long, 5> key = {pr->g.nx, pr->g.ny, pr->g.nz, pr->solver,
-                                        pr->prm.boundary_method};
-  auto hit = tuned.find(key);
-  if (hit != tuned.end()) {
-    pr->coop_threads = hit->second;
-    pr->coop_blocks = 0;
-    return PM_OK;
-  }
-  static const int cand[] = {256, 128, 64, 32};
-  float best = 1e30f;
-  int bt = 256;
-  for (int t : cand) {
-    int blocks = 0;
-    CK(launch_wavefront(pr->F[1], pr->codes, pr->g, pr->solver, 1, t, &blocks, pr->st));
-    CK(cudaEventRecord(pr->ev0, pr->st));
-    CK(launch_wavefront(pr->F[1], pr->codes, pr->g, pr->solver, 2, t, &blocks, pr->st));
-    CK(cudaEventRecord(pr->ev1, pr->st));
-    pm_status s = device_sync(pr, "wavefront shape");
-    if (s != PM_OK) return s;
-    float ms = 0.f;
-    CK(cudaEventElapsedTime(&ms, pr->ev0, pr->ev1));
-    if (ms < 0.98f * best) { best = ms; bt = t; }
-  }
-  CK(launch_copy_fields64(pr->F[1], pr->F[0], pr->g, pr->st));
-  pr->coop_threads = bt;
-  pr->coop_blocks = 0;
-  tuned[key] = bt;
-  return device_sync(pr, "wavefront shape");
-}
-
 pm_status dc_flush(pm_problem* pr) {
   if (pr->dc_pos > 0) {
     if (pr->compact())
@@ -543,8 +506,14 @@ namespace {
 
 pm_status iterate_direct(pm_problem* pr, int n) {
   for (int i = 0; i < n; ++i) {
-    pm_status s = pr->precision == PM_PREC_MIXED ? iterate_mixed(pr) : iterate64(pr);
-    if (s != PM_OK) return s;
+    if (pr->order == PM_ORDER_REFERENCE) {
+      // in place: the second state's memory is the sweep's exchange
+      CK(launch_wave(pr->F[0], pr->codes, pr->g, pr->solver, pr->f64_base[1], pr->werr,
+                     pr->st));
+    } else {
+      pm_status s = pr->precision == PM_PREC_MIXED ? iterate_mixed(pr) : iterate64(pr);
+      if (s != PM_OK) return s;
+    }
     pr->iteration++;
     pr->sweeps_done++;
   }
@@ -556,21 +525,13 @@ constexpr size_t kGraphCache = 8;
 
 }  // namespace
 
-// A block of n sweeps of the out-of-place orders runs as one CUDA graph: the
+// A block of n sweeps runs as one CUDA graph: the
 // first time a (length, parity state) occurs the launches are captured while
 // the host bookkeeping advances as usual, later blocks with the same start
 // state replay the graph and apply the recorded end state.  Graph launches
 // cut the per-kernel launch cost that dominates small domains.
 pm_status pm::iterate_n(pm_problem* pr, int n) {
   if (n <= 0) return PM_OK;
-  if (pr->order == PM_ORDER_REFERENCE) {
-    CK(launch_wavefront(pr->F[pr->cur], pr->codes, pr->g, pr->solver, n, pr->coop_threads,
-                        &pr->coop_blocks,
-                        pr->st));
-    pr->iteration += n;
-    pr->sweeps_done += n;
-    return PM_OK;
-  }
   // long runs go as it_eval-long chunks, whose graphs repeat
   const int chunk = std::max(kGraphMinSweeps, pr->prm.it_eval);
   while (n > chunk) {
@@ -782,6 +743,7 @@ pm_status pm_problem_footprint(const pm_params* p, size_t* bytes) {
 pm_status pm_debug_tma_fail(int on) {
   zmarch_debug_fail(on);
   compact_debug_fail(on);
+  wave_debug_fail(on);
   return PM_OK;
 }
 
@@ -869,6 +831,7 @@ pm_status pm::problem_create(const pm_params* p, const uint8_t* geom, int rot_ax
     const size_t o_part = c.take(sizeof(double) * kRedBlocks * kRedVals + 64);
     const size_t o_dout = c.take(sizeof(double) * 16);
     const size_t o_scr = c.take(pr->scratch_bytes);
+    const size_t o_werr = c.take(sizeof(int));
     CKF(dev_alloc((void**)&pr->arena, c.bytes));
     char* a = (char*)pr->arena;
     pr->codes_base = (uint8_t*)(a + o_codes);
@@ -877,6 +840,10 @@ pm_status pm::problem_create(const pm_params* p, const uint8_t* geom, int rot_ax
     pr->partials = (double*)(a + o_part);
     pr->dout = (double*)(a + o_dout);
     pr->scratch = a + o_scr;
+    if (pr->order == PM_ORDER_REFERENCE) {
+      pr->werr = (int*)(a + o_werr);
+      CKF(cudaMemsetAsync(pr->werr, 0, sizeof(int), pr->st));
+    }
   }
   pr->codes = pr->codes_base + kXoffC;
   CKF(cudaMemsetAsync(pr->codes_base, 0, g.allocc, pr->st));
@@ -966,10 +933,7 @@ pm_status pm::problem_create(const pm_params* p, const uint8_t* geom, int rot_ax
     pm_status ts = choose_correction_kernel(pr, p->kernel);
     if (ts != PM_OK) return fail(ts);
   }
-  if (pr->order == PM_ORDER_REFERENCE) {
-    pm_status ts = choose_wavefront_shape(pr);
-    if (ts != PM_OK) return fail(ts);
-  } else if (pr->precision == PM_PREC_FP64) {
+  if (pr->precision == PM_PREC_FP64 && pr->order != PM_ORDER_REFERENCE) {
     pm_status ts = choose_fp64_shapes(pr);
     if (ts != PM_OK) return fail(ts);
   }

@@ -109,8 +109,7 @@ struct pm_problem {
   double* hout = nullptr;  // pinned (a 256-byte slot of the process-wide pool)
   void* scratch = nullptr;  // export buffer
   size_t scratch_bytes = 0;
-  int coop_blocks = 0;
-  int coop_threads = 256;  // block size of the reference-order wavefront
+  int* werr = nullptr;  // reference order: a wait of the sweep ran out
   pm::ZmarchPlan* zp = nullptr;  // TMA z-march plan of the mixed form
   pm::BrickPlan* bp = nullptr;   // TMA brick plan of the mixed form
   int kern = 1;                  // correction-sweep kernel in use (see choose_correction_kernel)

@@ -93,11 +93,12 @@ cudaError_t launch_copy_fields64(Fields<double> dst, Fields<double> src, const G
 cudaError_t launch_halo64(Fields<double> f, const Grid& g, cudaStream_t st);
 cudaError_t launch_reapply64(double* p, const uint8_t* codes, const Grid& g, cudaStream_t st);
 
-// Reference order: in-place lexicographic sweep as an exact hyperplane
-// wavefront, then halo exchange and reapply, n_iter times (cooperative launch).
-cudaError_t launch_wavefront(Fields<double> f, const uint8_t* codes, const Grid& g,
-                             int solver, int n_iter, int threads, int* coop_blocks,
-                             cudaStream_t st);
+// Reference order (pm_wave.cu): one in-place lexicographic sweep, then halo
+// exchange and reapply.  exchange: 4 alloc64 doubles, its contents lost; err:
+// set when a bounded wait ran out.
+cudaError_t launch_wave(Fields<double> f, const uint8_t* codes, const Grid& g, int solver,
+                        double* exchange, int* err, cudaStream_t st);
+void wave_debug_fail(int on);
 
 // Ping-pong Jacobi (phase 0) and red (1) / black (2) half-sweeps from A into B
 // over the fluid list; periodic halo copies and the pressure reapply fused.

@@ -2,15 +2,11 @@
 // This translation unit is compiled with -fmad=false so that every
 // floating-point expression rounds exactly as the reference CPU program's
 // (which is built for x86-64 without FMA contraction).
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <atomic>
 
 #include "pm_internal.h"
 #include "pm_stencil.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace pm {
 
@@ -462,78 +458,6 @@ cudaError_t launch_reapply64(double* p, const uint8_t* codes, const Grid& g, cud
   k_reapply64<<<148, 256, 0, st>>>(p, codes, g);
   count_launches(1);
   return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------ reference order
-template <int SOLVER>
-__global__ void __launch_bounds__(256) k_wavefront(Fields<double> f, const uint8_t* codes, Grid g,
-                                                   int n_iter) {
-  cg::grid_group grid = cg::this_grid();
-  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nth = (long long)gridDim.x * blockDim.x;
-  const long long px = g.px64, pl = g.pl64;
-  const int T = g.nx + g.ny + g.nz - 2;
-  const long long nhalo =
-      4LL * ((long long)g.ny * g.nz + (long long)g.nx * g.nz + (long long)g.nx * g.ny);
-  for (int it = 0; it < n_iter; ++it) {
-    // central_diff5's lexicographic in-place order is reproduced exactly by
-    // hyperplanes t = x'+y'+z': every read at offsets -1/-2 lies on t-1/t-2
-    // (already updated), every read at +1/+2 on t+1/t+2 (not yet updated).
-    for (int t = 0; t < T; ++t) {
-      int zlo = max(0, t - (g.nx - 1) - (g.ny - 1)), zhi = min(g.nz - 1, t);
-      long long npairs = (long long)(zhi - zlo + 1) * g.ny;
-      for (long long q = tid; q < npairs; q += nth) {
-        int zp = zlo + (int)(q / g.ny), yp = (int)(q % g.ny);
-        int xp = t - zp - yp;
-        if (xp < 0 || xp >= g.nx) continue;
-        int x = xp + 2, y = yp + 2, z = zp + 2;
-        int code = codes[((long long)z * g.NY + y) * g.pxc + x];
-        if (!code) continue;
-        long long c = (long long)z * pl + (long long)y * px + x;
-        Stencil<double> s;
-        gather<double, 0, false, 0>(s, f, f, c, x, y, z, g, px, pl);
-        double un, vn, wn, pn;
-        update_exact<SOLVER>(s, code, un, vn, wn, pn);
-        f.u[c] = un;
-        f.v[c] = vn;
-        f.w[c] = wn;
-        f.p[c] = pn;
-      }
-      grid.sync();
-    }
-    for (long long q = tid; q < nhalo; q += nth) halo_point<double>(f, g, px, pl, q);
-    grid.sync();
-    for (long long q = tid; q < (long long)g.nx * g.ny; q += nth) reapply_point(f.p, codes, g, q);
-    grid.sync();
-  }
-}
-
-// threads: block size (32..256).  The grid holds one thread per (y, z) pair
-// of a hyperplane -- enough for any hyperplane -- as far as co-residency
-// allows; smaller blocks spread the same threads over more SMs (more FP64
-// throughput per hyperplane, a dearer grid barrier).
-cudaError_t launch_wavefront(Fields<double> f, const uint8_t* codes, const Grid& g, int solver,
-                             int n_iter, int threads, int* coop_blocks, cudaStream_t st) {
-  void* fn = solver == 1 ? (void*)k_wavefront<1> : solver == 2 ? (void*)k_wavefront<2>
-                                                               : (void*)k_wavefront<3>;
-  if (threads < 32 || threads > 256) threads = 256;
-  if (*coop_blocks <= 0) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, 0);
-    if (e != cudaSuccess) return e;
-    long long want = ((long long)g.ny * g.nz + threads - 1) / threads;
-    long long maxb = (long long)sms * (per > 0 ? per : 1);
-    *coop_blocks = (int)(want < maxb ? (want < 1 ? 1 : want) : maxb);
-  }
-  Fields<double> ff = f;
-  const uint8_t* cc = codes;
-  Grid gg = g;
-  int n = n_iter;
-  void* args[] = {&ff, &cc, &gg, &n};
-  count_launches(1);
-  return cudaLaunchCooperativeKernel(fn, dim3(*coop_blocks), dim3(threads), args, 0, st);
 }
 
 // ------------------------------------------------------------------ FP64 sweeps (exact)

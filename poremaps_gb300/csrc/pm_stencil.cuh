@@ -54,6 +54,35 @@ __device__ __forceinline__ double d2_exact(int cs, double ll, double l, double m
   return d;
 }
 
+// Whether x is +0 or -0, without the FP64 pipe.
+__device__ __forceinline__ bool zero_bits(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+
+// x / kRe, correctly rounded, in three FP64 instructions instead of the
+// general division: kInvRe is the correctly rounded reciprocal, x * kInvRe is
+// less than an ulp from the quotient (the reciprocal is off by 0.19 of half an
+// ulp, the product by half an ulp), and one residual step then rounds
+// correctly (Markstein 1990; Brisebarre, Muller and Raina, IEEE TC 53, 2004).
+// The step needs the residual exact and the product finite; arguments for
+// which that is not sure take the division.  Zero, whose sign the step would
+// lose, is its own quotient.
+__device__ __forceinline__ double div_re_step(double x) {
+  constexpr double kInvRe = 1.0 / kRe;
+  static_assert(kRe == 0.01, "the product's error bound above is for this divisor");
+  const double q = x * kInvRe;
+  const double r = __fma_rn(__fma_rn(-kRe, q, x), kInvRe, q);
+  return zero_bits(x) ? x : r;
+}
+__device__ __forceinline__ bool div_re_holds(double x) {
+  return zero_bits(x) || (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 64u < 1900u;
+}
+__device__ __noinline__ static double div_re_general(double x) { return x / kRe; }
+__device__ __forceinline__ double div_re(double x) {
+  const double r = div_re_step(x);
+  return div_re_holds(x) ? r : div_re_general(x);
+}
+
 // central_diff5 body (src/solver.cc:142-219) for one fluid voxel.
 template <int SOLVER>
 __device__ __forceinline__ void update_exact(const Stencil<double>& s, int code, double& un,
@@ -79,13 +108,13 @@ __device__ __forceinline__ void update_exact(const Stencil<double>& s, int code,
   double v_sum = 0.0;
   if (SOLVER == 1) v_sum = (s.wzp - s.wc + s.vyp - s.vc + s.uxp - s.uc);
   if (SOLVER == 1 || SOLVER == 2) {
-    un = lx ? 0.0 : s.uc + (-dp_dx + fu / kRe) * kDt;
-    vn = ly ? 0.0 : s.vc + (-dp_dy + fv / kRe) * kDt;
-    wn = lz ? 0.0 : s.wc + (-dp_dz + fw / kRe) * kDt;
+    un = lx ? 0.0 : s.uc + (-dp_dx + div_re(fu)) * kDt;
+    vn = ly ? 0.0 : s.vc + (-dp_dy + div_re(fv)) * kDt;
+    wn = lz ? 0.0 : s.wc + (-dp_dz + div_re(fw)) * kDt;
   } else {
-    un = (1.0 - kOmega) * s.uc + kOmega * (-dp_dx + fu / kRe) * kDt;
-    vn = (1.0 - kOmega) * s.vc + kOmega * (-dp_dy + fv / kRe) * kDt;
-    wn = (1.0 - kOmega) * s.wc + kOmega * (-dp_dz + fw / kRe) * kDt;
+    un = (1.0 - kOmega) * s.uc + kOmega * (-dp_dx + div_re(fu)) * kDt;
+    vn = (1.0 - kOmega) * s.vc + kOmega * (-dp_dy + div_re(fv)) * kDt;
+    wn = (1.0 - kOmega) * s.wc + kOmega * (-dp_dz + div_re(fw)) * kDt;
   }
   if (SOLVER == 2 || SOLVER == 3) v_sum = (s.wzp - wn + s.vyp - vn + s.uxp - un);
   pn = s.pc - kC2 * v_sum * kDt;
