@@ -585,8 +585,8 @@ namespace {
 pm_status reduce_launch(pm_problem* pr, int full) {
   int mode = (pr->precision == PM_PREC_MIXED && pr->dc_pos > 0) ? 1 : 0;
   if (pr->order == PM_ORDER_REFERENCE) {
-    CK(launch_reduce_serial(pr->F[pr->cur], full, pr->codes, pr->g, pr->prm.dom_interest,
-                            pr->dout, pr->st));
+    CK(launch_reduce_serial(pr->F[pr->cur], full, pr->list, pr->nlist, pr->g,
+                            pr->prm.dom_interest, pr->dout, pr->st));
     CK(cudaMemcpyAsync(pr->hout, pr->dout, sizeof(double) * kRedVals, cudaMemcpyDeviceToHost,
                        pr->st));
     return PM_OK;

@@ -149,8 +149,8 @@ cudaError_t launch_reduce(Fields<double> x, const float4* e, int mode, int full,
 
 // The same sums in the reference's serial lexicographic order (bitwise equal
 // to the reference's reductions; used by the reference order).
-cudaError_t launch_reduce_serial(Fields<double> x, int full, const uint8_t* codes, const Grid& g,
-                                 const int di[6], double* out, cudaStream_t st);
+cudaError_t launch_reduce_serial(Fields<double> x, int full, const int* list, int nlist,
+                                 const Grid& g, const int di[6], double* out, cudaStream_t st);
 
 cudaError_t launch_pack64(const double* f, const uint8_t* codes, int implied3, const Grid& g,
                           double* out, cudaStream_t st);
