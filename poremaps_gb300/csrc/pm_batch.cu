@@ -9,6 +9,10 @@
 // The mixed form's correction and residual are the compact store of
 // pm_compact.cu (one float4 per fluid-list position), as the single-problem
 // kernel 8 uses them.
+#include <stddef.h>
+
+#include <algorithm>
+
 #include "pm_batch.h"
 #include "pm_compact.cuh"
 
@@ -88,6 +92,55 @@ __global__ void __launch_bounds__(512, 2)
     float4* Eout = a ? sd.E0 : sd.E1;
     batch_inner_voxel<S, false>(sd, Ein, Eout, q);
   });
+}
+
+// One correction sweep over flat items: as the single problem's sweep over
+// packed records (k_dc_inner_cr), 1024 threads per SM, the next record in
+// flight while a voxel is computed, launches overlapping.  A block's items are
+// staged in shared memory before the wait for the previous sweep.
+// Bound as that sweep is: 92 voxels per ns on six samples of 5.8M fluid voxels
+// (63 us a sweep).  Against the tile queue of k_batch_inner_round, whose
+// fences and tickets it does without: 76 -> 64 ms for 24 samples of 32..128, 112
+// -> 92 ms for six of 96..192, 0.32 -> 0.19 ms a block for two of 12^3.
+constexpr int kFlatStage = 32;
+static_assert(offsetof(FlatSample, start) == 48 && sizeof(FlatSample) == 64, "staged by quads");
+template <int S>
+__global__ void __launch_bounds__(kFlatVoxels, 4)
+    k_batch_flat(const FlatSample* __restrict__ samples, const int2* __restrict__ items,
+                 int nitems, int round) {
+  __shared__ FlatSample sh[kFlatStage];
+  const int tid = threadIdx.x, G = gridDim.x, a = (round - 1) & 1;
+  auto record = [&](const FlatSample& it) {
+    return ld_record(it.rec + min(it.start + tid, it.nlist - 1));
+  };
+  uint4 rc = make_uint4(0u, 0u, 0u, 0u);
+  for (int base = blockIdx.x; base < nitems; base += kFlatStage * G) {
+    const int n = min(kFlatStage, (nitems - base + G - 1) / G);
+    __syncthreads();  // every reader of the previous items is done
+    constexpr int W = sizeof(FlatSample) / 16;
+    for (int i = tid; i < n * W; i += kFlatVoxels) {
+      const int2 it = __ldg(items + base + (long long)(i / W) * G);
+      uint4 v = __ldg(reinterpret_cast<const uint4*>(samples + it.x) + i % W);
+      if (i % W == W - 1) v.x = it.y;  // start
+      reinterpret_cast<uint4*>(sh)[i] = v;
+    }
+    __syncthreads();
+    rc = record(sh[0]);
+    if (base == blockIdx.x) asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int j = 0; j < n; ++j) {
+      const FlatSample& it = sh[j];
+      if (base + (j + 1) * G >= nitems) asm volatile("griddepcontrol.launch_dependents;");
+      const uint4 next = record(sh[min(j + 1, n - 1)]);
+      const int q = it.start + tid;
+      if (q < it.nlist) {
+        if ((S ? S : it.solver) == 3)
+          inner_r_voxel<3>(it.E[a], it.E[1 - a], it.R, rc, it.ya, q, it.nlist);
+        else
+          inner_r_voxel<2>(it.E[a], it.E[1 - a], it.R, rc, it.ya, q, it.nlist);
+      }
+      rc = next;
+    }
+  }
 }
 
 __global__ void k_batch_correct(const SampleDesc* d, const WorkItem* items, int nitems,
@@ -240,6 +293,15 @@ cudaError_t launch_batch_round(const SampleDesc* d, const WorkItem* items, int n
     k_batch_inner_round<0><<<grid, threads, 0, st>>>(d, items, nitems, sweeps, sync, extra, polls);
   count_launches(1);
   return cudaGetLastError();
+}
+
+cudaError_t launch_batch_flat(const FlatSample* samples, const int2* items, int nitems, int round,
+                              int solver, cudaStream_t st) {
+  if (nitems <= 0) return cudaSuccess;
+  const int blocks = std::min(nitems, 1024 / kFlatVoxels * sm_count());
+  count_launches(1);
+  auto* k = solver == 2 ? k_batch_flat<2> : solver == 3 ? k_batch_flat<3> : k_batch_flat<0>;
+  return launch_overlapped(k, blocks, kFlatVoxels, st, samples, items, nitems, round);
 }
 
 cudaError_t launch_batch(int kind, const SampleDesc* d, const WorkItem* items, int nitems,

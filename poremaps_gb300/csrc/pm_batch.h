@@ -32,6 +32,19 @@ struct WorkItem {
   int sample_items;  // items of the same sample in the table
 };
 
+// One sample as the correction sweeps over packed records see it; a flat item
+// is kFlatVoxels fluid-list positions of a sample, from .y.
+constexpr int kFlatVoxels = 256;
+struct alignas(16) FlatSample {
+  float4* E[2];
+  const float4* R;
+  const uint4* rec;
+  const int2* ya;
+  int nlist, solver;
+  int start;  // of the item, in the kernel's copy
+  int pad[3];
+};
+
 enum { kBatchResidual = 0, kBatchInner = 1, kBatchCorrect = 2, kBatchSweep64 = 3, kBatchSumW = 4 };
 
 // kind: kBatch*; round: sweep index inside the block (inner / sweep64), the
@@ -41,6 +54,11 @@ enum { kBatchResidual = 0, kBatchInner = 1, kBatchCorrect = 2, kBatchSweep64 = 3
 cudaError_t launch_batch(int kind, const SampleDesc* d, const WorkItem* items, int nitems,
                          int round, int threads, int blocks, double* out, cudaStream_t st,
                          int solver = 0);
+
+// Correction sweep `round` (1 ..) over the flat items of one or more samples
+// whose first residual wrote E[0].
+cudaError_t launch_batch_flat(const FlatSample* samples, const int2* items, int nitems, int round,
+                              int solver, cudaStream_t st);
 
 // The FP32 correction sweeps 1 .. sweeps of a round (mixed form) in one
 // persistent launch walking a device tile queue: CTAs take tickets (sweep k,

@@ -362,23 +362,6 @@ cudaError_t compact_records(const unsigned* meta, const int4* sa, const int2* sb
   return cudaGetLastError();
 }
 
-// A launch whose CTAs may become resident before the stream's previous kernel
-// has ended (they wait for it themselves).
-template <typename... P, typename... A>
-static cudaError_t launch_overlapped(void (*kernel)(P...), int blocks, int threads,
-                                     cudaStream_t st, A... args) {
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((unsigned)blocks);
-  c.blockDim = dim3((unsigned)threads);
-  c.stream = st;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, args...);
-}
-
 template <int THREADS>
 static cudaError_t inner_cr_launch(const float4* e, float4* e2, const float4* r, const uint4* rec,
                                    const int2* ya, int nlist, int solver, cudaStream_t st) {

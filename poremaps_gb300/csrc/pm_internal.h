@@ -158,4 +158,23 @@ cudaError_t launch_unpack64(const double* in, const Grid& g, double* f, cudaStre
 cudaError_t launch_pack_codes(const uint8_t* codes, const Grid& g, int* out, cudaStream_t st);
 
 
+#ifdef __CUDACC__
+// A launch whose CTAs may become resident before the stream's previous kernel
+// has ended (they wait for it themselves, griddepcontrol.wait).
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), int blocks, int threads, cudaStream_t st,
+                              A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
+#endif
+
 }  // namespace pm

@@ -10,9 +10,10 @@
 //      evaluates convergence after the sweeps it_eval, 2 it_eval, ...);
 //   2. runs one it_eval block for all resident samples over a work table of
 //      (sample, fluid-voxel run) items: the FP64 residual, the it_eval - 1
-//      FP32 correction sweeps as one persistent kernel walking a device tile
-//      queue (or one launch per sweep), the FP64 correction and a per-item sum
-//      of w, captured once per change of the resident set in a CUDA graph;
+//      FP32 correction sweeps as overlapped launches over packed records (or
+//      one persistent kernel walking a device tile queue, or plain launches),
+//      the FP64 correction and a per-item sum of w, captured once per change
+//      of the resident set in a CUDA graph;
 //   3. evaluates compute_convergence per sample (the reference's stop rule)
 //      and retires the finished ones (permeability, completion record,
 //      device memory freed) without touching the others.
@@ -80,6 +81,12 @@ struct pm_server {
   size_t cap_desc = 0;
   WorkItem* d_items = nullptr;
   size_t cap_items = 0;
+  std::vector<FlatSample> h_fsamp;  // the sweeps over packed records: samples,
+  std::vector<int2> h_flat;         // their items (sample, first position; or empty)
+  std::vector<std::pair<int, int>> flat_group;  // first item and count of each group
+  FlatSample* d_fsamp = nullptr;
+  int2* d_flat = nullptr;
+  size_t cap_fsamp = 0, cap_flat = 0;
   double* d_part = nullptr;
   double* h_part = nullptr;
   size_t cap_part = 0;
@@ -100,11 +107,6 @@ struct pm_server {
 };
 
 namespace {
-
-// pm_debug_round_wait: added to every wait target of the persistent round,
-// and its poll limit (0 = the kernel's own).
-std::atomic<unsigned> g_round_extra{0};
-std::atomic<int> g_round_polls{0};
 
 double now_ms(pm_server* s) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - s->t0)
@@ -281,6 +283,59 @@ void build_items(pm_server* s, int chunk) {
   }
 }
 
+bool mixed(const pm_server* s) { return s->cfg.precision == PM_PREC_MIXED; }
+
+// pm_debug_round_wait: added to every wait target of the persistent round,
+// and its poll limit (0 = the kernel's own).
+std::atomic<unsigned> g_round_extra{0};
+std::atomic<int> g_round_polls{0};
+
+// Whether a block's correction sweeps run over flat items, one overlapped
+// launch per sweep.  Faster than the persistent round over its tile queue at
+// every size measured (1.4k to 5.8M fluid voxels, see k_batch_flat), so that
+// one is left for media whose offsets the packed records do not hold, for a
+// launch shape set by the caller, and for its test hook.
+bool flat_sweeps(const pm_server* s) {
+  if (!mixed(s) || s->cfg.relaunch_sweeps || s->shape_pinned || s->block < 2 ||
+      g_round_extra.load() || g_round_polls.load())
+    return false;
+  for (auto& r : s->res)
+    if (!r.pr->crec) return false;
+  return true;
+}
+
+// Sweeps run group by group: whole samples whose e, r and records (64 bytes a
+// voxel) L2 holds together, so that all sweeps of a block but the first read
+// them there.  Six samples of 5.8M voxels: 92 ms at 100 and 130 MB a group, 97
+// at 40, 96 in one group; 24 of 32..128: 64 ms at 130, 71 at 60, 97 at 20,
+// where groups are too small for the device, 65 in one.
+constexpr size_t kGroupBytes = 128u << 20;
+
+void build_flat(pm_server* s) {
+  size_t bytes = 0;
+  for (size_t i = 0; i < s->res.size(); ++i) {
+    const pm_problem* pr = s->res[i].pr;
+    const size_t b = (size_t)pr->nlist * (3 * sizeof(float4) + sizeof(uint4));
+    if (s->flat_group.empty() || bytes + b > kGroupBytes) {
+      s->flat_group.push_back({(int)s->h_flat.size(), 0});
+      bytes = 0;
+    }
+    bytes += b;
+    FlatSample d;
+    memset(&d, 0, sizeof d);
+    d.E[0] = pr->Ec[0];
+    d.E[1] = pr->Ec[1];
+    d.R = pr->Rc;
+    d.rec = pr->crec;
+    d.ya = pr->cslot2;
+    d.nlist = pr->nlist;
+    d.solver = pr->solver;
+    s->h_fsamp.push_back(d);
+    for (int a = 0; a < pr->nlist; a += kFlatVoxels) s->h_flat.push_back(make_int2((int)i, a));
+    s->flat_group.back().second = (int)s->h_flat.size() - s->flat_group.back().first;
+  }
+}
+
 pm_status upload(pm_server* s) {
   pm_status e;
   if ((e = grow(&s->d_desc, &s->cap_desc, s->h_desc.size())) != PM_OK) return e;
@@ -298,13 +353,19 @@ pm_status upload(pm_server* s) {
   }
   SCK(cudaMemcpyAsync(s->d_desc, s->h_desc.data(), s->h_desc.size() * sizeof(SampleDesc),
                       cudaMemcpyHostToDevice, s->st));
+  if (!s->h_flat.empty()) {
+    if ((e = grow(&s->d_fsamp, &s->cap_fsamp, s->h_fsamp.size())) != PM_OK) return e;
+    if ((e = grow(&s->d_flat, &s->cap_flat, s->h_flat.size())) != PM_OK) return e;
+    SCK(cudaMemcpyAsync(s->d_fsamp, s->h_fsamp.data(), s->h_fsamp.size() * sizeof(FlatSample),
+                        cudaMemcpyHostToDevice, s->st));
+    SCK(cudaMemcpyAsync(s->d_flat, s->h_flat.data(), s->h_flat.size() * sizeof(int2),
+                        cudaMemcpyHostToDevice, s->st));
+  }
   SCK(cudaMemcpyAsync(s->d_items, s->h_items.data(), s->h_items.size() * sizeof(WorkItem),
                       cudaMemcpyHostToDevice, s->st));
   SCK(cudaStreamSynchronize(s->st));
   return PM_OK;
 }
-
-bool mixed(const pm_server* s) { return s->cfg.precision == PM_PREC_MIXED; }
 
 // The launches of one block (recorded into a graph or issued directly).
 pm_status issue_block(pm_server* s, int* nk) {
@@ -314,7 +375,11 @@ pm_status issue_block(pm_server* s, int* nk) {
     SCK(launch_batch(kBatchResidual, s->d_desc, s->d_items, n, 0, T, 0, nullptr, s->st,
                      s->solver));
     ++k;
-    if (s->cfg.relaunch_sweeps) {
+    if (!s->h_flat.empty()) {
+      for (auto& g : s->flat_group)
+        for (int r = 1; r < s->block; ++r, ++k)
+          SCK(launch_batch_flat(s->d_fsamp, s->d_flat + g.first, g.second, r, s->solver, s->st));
+    } else if (s->cfg.relaunch_sweeps) {
       for (int r = 1; r < s->block; ++r, ++k)
         SCK(launch_batch(kBatchInner, s->d_desc, s->d_items, n, r, T, 0, nullptr, s->st,
                          s->solver));
@@ -498,7 +563,12 @@ pm_status rebuild(pm_server* s) {
     s->h_desc.push_back(d);
   }
   pm_status e;
-  if (s->cfg.autotune && !s->shape_pinned && (e = autotune(s)) != PM_OK) return e;
+  s->h_fsamp.clear();
+  s->h_flat.clear();
+  s->flat_group.clear();
+  const bool flat = flat_sweeps(s);
+  if (!flat && s->cfg.autotune && !s->shape_pinned && (e = autotune(s)) != PM_OK) return e;
+  if (flat) build_flat(s);
   build_items(s, s->chunk);
   if ((e = upload(s)) != PM_OK) return e;
   drop_graph(s);
@@ -533,7 +603,8 @@ pm_status run_block(pm_server* s) {
   }
   SCK(cudaMemcpyAsync(s->h_part, s->d_part, s->h_items.size() * sizeof(double),
                       cudaMemcpyDeviceToHost, s->st));
-  const bool round = mixed(s) && !s->cfg.relaunch_sweeps && s->block > 1;
+  const bool round =
+      mixed(s) && !s->cfg.relaunch_sweeps && s->block > 1 && s->h_flat.empty();
   if (round)
     SCK(cudaMemcpyAsync(s->h_flag, s->d_sync + 1, sizeof(unsigned), cudaMemcpyDeviceToHost,
                         s->st));
@@ -622,6 +693,8 @@ pm_status pm_server_destroy(pm_server* s) {
   drop_graph(s);
   cudaFree(s->d_desc);
   cudaFree(s->d_items);
+  cudaFree(s->d_fsamp);
+  cudaFree(s->d_flat);
   cudaFree(s->d_part);
   cudaFree(s->d_sync);
   if (s->h_part) cudaFreeHost(s->h_part);
