@@ -221,11 +221,11 @@ pm_status iterate64(pm_problem* pr) {
   return PM_OK;
 }
 
-// Launch form of each FP64 phase (persistent or one voxel per thread), timed
-// on the problem: the persistent form wins on porous media at 128^3, the
-// one-voxel form can win where a phase needs more registers than the
-// persistent launch allows.  Both give identical fields; the trials sweep
-// the initial state into the second buffer, which is restored afterwards.
+// Launch form of each FP64 phase (persistent with 2 or 3 CTAs per SM, or one
+// voxel per thread), timed on the problem: the lists' lengths decide how evenly
+// the waves of each form end (a 97x61x118 pack sweeps in 21.9 us with 2 CTAs
+// per SM and 25.7 with 3, a 128^3 one in 59.8 and 57.6).  All give identical
+// fields; the trials sweep the two states, which are set up again afterwards.
 pm_status choose_fp64_shapes(pm_problem* pr) {
   if (pr->exact) return PM_OK;
   static std::mutex mu;
@@ -239,30 +239,27 @@ pm_status choose_fp64_shapes(pm_problem* pr) {
     for (int i = 0; i < 3; ++i) pr->pf64[i] = hit->second[i];
     return PM_OK;
   }
-  const Fields<double> A = pr->F[0], B = pr->F[1];
-  const int phases[2] = {pr->order == PM_ORDER_JACOBI ? 0 : 1, 2};
-  const int nph = pr->order == PM_ORDER_JACOBI ? 1 : 2;
-  for (int k = 0; k < nph; ++k) {
-    const int ph = phases[k];
-    const int* list = ph == 2 ? pr->list + pr->nred : pr->list;
-    const int n = ph == 0 ? pr->nlist : ph == 1 ? pr->nred : pr->nlist - pr->nred;
-    float t[2] = {1e30f, 1e30f};
-    for (int form = 1; form >= 0; --form) {
-      CK(launch_sweep64(A, B, pr->codes, list, n, pr->g, pr->solver, 0, ph, pr->st, form));
-      for (int trial = 0; trial < 3; ++trial) {
-        CK(cudaEventRecord(pr->ev0, pr->st));
-        for (int r = 0; r < 3; ++r)
-          CK(launch_sweep64(A, B, pr->codes, list, n, pr->g, pr->solver, 0, ph, pr->st, form));
-        CK(cudaEventRecord(pr->ev1, pr->st));
-        pm_status s = device_sync(pr, "FP64 sweep shape");
-        if (s != PM_OK) return s;
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, pr->ev0, pr->ev1));
-        if (ms < t[form]) t[form] = ms;
-      }
+  // whole iterations in turn between the two states, as a solve runs them
+  auto set = [&](int form) { for (int& f : pr->pf64) f = form; };
+  float t[3] = {1e30f, 1e30f, 1e30f};
+  for (int form = 2; form >= 0; --form) {
+    set(form);
+    pm_status s = iterate64(pr);
+    for (int trial = 0; trial < 2 && s == PM_OK; ++trial) {
+      CK(cudaEventRecord(pr->ev0, pr->st));
+      for (int r = 0; r < 4 && s == PM_OK; ++r) s = iterate64(pr);
+      CK(cudaEventRecord(pr->ev1, pr->st));
+      if (s == PM_OK) s = device_sync(pr, "FP64 sweep shape");
+      float ms = 0.f;
+      if (s == PM_OK) CK(cudaEventElapsedTime(&ms, pr->ev0, pr->ev1));
+      t[form] = std::min(t[form], ms);
     }
-    pr->pf64[ph] = t[0] < 0.98f * t[1] ? 0 : 1;
+    if (s != PM_OK) return s;
   }
+  const int pf = t[2] < t[1] ? 2 : 1;
+  set(t[0] < 0.98f * t[pf] ? 0 : pf);
+  pr->cur = 0;
+  CK(launch_init64(pr->F[0], pr->codes, pr->g, pr->st));
   CK(launch_copy_fields64(pr->F[1], pr->F[0], pr->g, pr->st));
   tuned[key] = {pr->pf64[0], pr->pf64[1], pr->pf64[2]};
   return device_sync(pr, "FP64 sweep shape");

@@ -188,8 +188,8 @@ template <int SOLVER>
 __global__ void __launch_bounds__(256, 2) k_dc_residual_c(Fields<double> X, float4* R,
                                                         float4* E, const uint8_t* codes,
                                                         const int* list, int nlist, Grid g) {
-  __shared__ double ctab[16];
-  fill_centre_table<SOLVER>(ctab);
+  __shared__ Tables64 tab;
+  fill_tables64<SOLVER>(tab);
   __syncthreads();
   const int stride = gridDim.x * blockDim.x;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256, 2) k_dc_residual_c(Fields<double> X, floa
   for (; q < nlist; q += stride) {
     const int qn = q + stride;
     const int next = qn < nlist ? __ldg(list + qn) : 0;
-    residual_c_voxel<SOLVER>(X, R, E, codes, g, q, lin, ctab);
+    residual_c_voxel<SOLVER>(X, R, E, codes, g, q, lin, &tab);
     lin = next;
   }
 }

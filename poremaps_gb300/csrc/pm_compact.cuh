@@ -360,17 +360,16 @@ __device__ __forceinline__ void inner_c_voxel(const float4* __restrict__ E,
 template <int SOLVER>
 __device__ __forceinline__ void residual_c_voxel(const Fields<double>& X, float4* R, float4* E,
                                                  const uint8_t* codes, const Grid& g, int q,
-                                                 int lin, const double* ctab = nullptr) {
+                                                 int lin, const Tables64* tab = nullptr) {
   int x, y, z;
   lin_to_xyz(lin, g, x, y, z);
   const int code = codes[((long long)z * g.NY + y) * g.pxc + x];
   const long long c = (long long)z * g.pl64 + (long long)y * g.px64 + x;
-  Stencil<double> s;
-  gather<double, 0>(s, X, X, c, x, y, z, g, g.px64, g.pl64);
+  Own64 o;
   double un, vn, wn, pn;
-  update_fast<double, SOLVER>(s, code, un, vn, wn, pn, ctab);
-  const double pstored = (z == g.NZ - 3) ? __ldg(X.p + c) : s.pc;
-  const float4 rv = make_float4((float)(un - s.uc), (float)(vn - s.vc), (float)(wn - s.wc),
+  update64<SOLVER, 0, kLdNc>(X, X, c, x, y, z, g, code, tab, o, un, vn, wn, pn);
+  const double pstored = (z == g.NZ - 3) ? __ldg(X.p + c) : o.p;
+  const float4 rv = make_float4((float)(un - o.u), (float)(vn - o.v), (float)(wn - o.w),
                                 (float)(pn - pstored));
   R[q] = rv;
   E[q] = rv;

@@ -9,6 +9,8 @@
 // sweeps ends with the FP64 update x += e and a fresh FP64 residual, so FP32
 // rounding only ever touches the (shrinking) correction and the iterate
 // converges to the FP64 fixed point.
+#include <algorithm>
+
 #include "pm_internal.h"
 #include "pm_stencil.cuh"
 
@@ -19,50 +21,72 @@ template <int SOLVER, int PHASE>
 __global__ void __launch_bounds__(256) k_sweep64_fast(Fields<double> A, Fields<double> B,
                                                       const uint8_t* codes, const int* list,
                                                       int nlist, Grid g) {
-  __shared__ double ctab[16];
-  fill_centre_table<SOLVER>(ctab);
+  __shared__ Tables64 tab;
+  fill_tables64<SOLVER>(tab);
   __syncthreads();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nlist; q += gridDim.x * blockDim.x)
-    sweep64_voxel<SOLVER, PHASE, false>(A, B, codes, g, list[q], ctab);
+    sweep64_voxel<SOLVER, PHASE, false>(A, B, codes, g, list[q], &tab);
 }
 
 cudaError_t sweep64_exact(Fields<double> A, Fields<double> B, const uint8_t* codes,
                           const int* list, int nlist, const Grid& g, int solver, int phase,
                           cudaStream_t st);
 
-// Persistent form: one wave of two CTAs per SM walks the list with a grid
+// Persistent form: one wave of MINB CTAs per SM walks the list with a grid
 // stride, each thread loading its next list entry before it computes the
-// current voxel (the FP64 stencil needs ~110 registers: two CTAs fit).
-template <int SOLVER, int PHASE>
-__global__ void __launch_bounds__(256, 2) k_sweep64_pf(Fields<double> A, Fields<double> B,
+// current voxel.  Launches overlap: a CTA's slot goes to the next sweep's as it
+// ends, which loads its tables and first list entries and waits for this sweep
+// before it touches a field.
+// Bound: the FP64 pipe (31 instructions of a warp per voxel, 25 of them FMAs of
+// 16 clocks per SM and 6 others of 19: 40 us for the 734k voxels of a 128^3
+// pack) and, between a warp's instructions there, its loads; the half-sweeps
+// of that pack also miss L2 (their two states touch 120 MB).  Two CTAs leave
+// 128 registers, so that all of a voxel's loads are in flight at once; three
+// leave 80, no spills, and keep the pipe busier where there is enough work:
+// Jacobi on the 128^3 pack 44.0 us against 46.5 with two, red-black 57.6 against
+// 59.8; a 97x61x118 pack 25.7 against 21.9 (its half-sweeps are 1.2 waves of
+// three).  With the whole stencil loaded and plain launches: 48.4, 63 and 26.1.
+template <int SOLVER, int PHASE, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_sweep64_pf(Fields<double> A, Fields<double> B,
                                                       const uint8_t* codes, const int* list,
                                                       int nlist, Grid g) {
-  __shared__ double ctab[16];
-  fill_centre_table<SOLVER>(ctab);
+  __shared__ Tables64 tab;
+  fill_tables64<SOLVER>(tab);
   __syncthreads();
   const int stride = gridDim.x * blockDim.x;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   int lin = q < nlist ? __ldg(list + q) : 0;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (; q < nlist; q += stride) {
     const int qn = q + stride;
+    if (qn >= nlist) asm volatile("griddepcontrol.launch_dependents;");
     const int next = qn < nlist ? __ldg(list + qn) : 0;
-    sweep64_voxel<SOLVER, PHASE, false>(A, B, codes, g, lin, ctab);
+    sweep64_voxel<SOLVER, PHASE, false, kLdPlain>(A, B, codes, g, lin, &tab);
     lin = next;
   }
+}
+
+template <int SOLVER, int MINB>
+static cudaError_t sweep_pf(Fields<double> A, Fields<double> B, const uint8_t* codes,
+                            const int* list, int nlist, const Grid& g, int phase,
+                            cudaStream_t st) {
+  const int blocks = std::min((nlist + 255) / 256, MINB * sm_count());
+  auto* k = phase == 0 ? k_sweep64_pf<SOLVER, 0, MINB>
+                       : phase == 1 ? k_sweep64_pf<SOLVER, 1, MINB> : k_sweep64_pf<SOLVER, 2, MINB>;
+  count_launches(1);
+  return launch_overlapped(k, blocks, 256, st, A, B, codes, list, nlist, g);
 }
 
 template <int SOLVER>
 static cudaError_t sweep_fast_s(Fields<double> A, Fields<double> B, const uint8_t* codes,
                                 const int* list, int nlist, const Grid& g, int phase,
                                 int persistent, cudaStream_t st) {
-  int blocks = (nlist + 255) / 256;
+  const int blocks = (nlist + 255) / 256;
   if (blocks < 1) return cudaSuccess;
-  if (persistent) {
-    const int sms = sm_count();
-    if (blocks > 2 * sms) blocks = 2 * sms;
-    if (phase == 0) k_sweep64_pf<SOLVER, 0><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
-    else if (phase == 1) k_sweep64_pf<SOLVER, 1><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
-    else k_sweep64_pf<SOLVER, 2><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
+  if (persistent == 1) {
+    return sweep_pf<SOLVER, 2>(A, B, codes, list, nlist, g, phase, st);
+  } else if (persistent == 2) {
+    return sweep_pf<SOLVER, 3>(A, B, codes, list, nlist, g, phase, st);
   } else {
     if (phase == 0) k_sweep64_fast<SOLVER, 0><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
     else if (phase == 1) k_sweep64_fast<SOLVER, 1><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
@@ -108,8 +132,8 @@ __global__ void __launch_bounds__(256, 2) k_dc_residual(Fields<double> X, float4
                                                       const uint8_t* codes, const int* list,
                                                       int nlist, Grid g) {
   // persistent, next list entry prefetched (as the FP64 sweeps)
-  __shared__ double ctab[16];
-  fill_centre_table<SOLVER>(ctab);
+  __shared__ Tables64 tab;
+  fill_tables64<SOLVER>(tab);
   __syncthreads();
   const int stride = gridDim.x * blockDim.x;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -117,7 +141,7 @@ __global__ void __launch_bounds__(256, 2) k_dc_residual(Fields<double> X, float4
   for (; q < nlist; q += stride) {
     const int qn = q + stride;
     const int next = qn < nlist ? __ldg(list + qn) : 0;
-    dc_residual_voxel<SOLVER>(X, R, E, codes, g, lin, ctab);
+    dc_residual_voxel<SOLVER>(X, R, E, codes, g, lin, &tab);
     lin = next;
   }
 }

@@ -102,8 +102,8 @@ void wave_debug_fail(int on);
 
 // Ping-pong Jacobi (phase 0) and red (1) / black (2) half-sweeps from A into B
 // over the fluid list; periodic halo copies and the pressure reapply fused.
-// persistent: one wave of 2 CTAs per SM walking the list (else one voxel per
-// thread); both give identical fields.
+// persistent: 1, 2: one wave of 2 / 3 CTAs per SM walking the list (0: one voxel
+// per thread); all give identical fields.
 cudaError_t launch_sweep64(Fields<double> A, Fields<double> B, const uint8_t* codes,
                            const int* list, int nlist, const Grid& g, int solver, int exact,
                            int phase, cudaStream_t st, int persistent = 1);
