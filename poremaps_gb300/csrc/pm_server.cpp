@@ -669,6 +669,7 @@ pm_status pm_server_create(const pm_server_config* cfg, pm_server** out) {
   if (s->cfg.max_resident <= 0) s->cfg.max_resident = 1024;
   size_t fr = 0, tot = 0;
   cudaError_t e = cudaMemGetInfo(&fr, &tot);
+  fr += pool_bytes();
   if (e != cudaSuccess) {
     delete s;
     return cuda_error(e, "cudaMemGetInfo");
