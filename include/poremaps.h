@@ -55,7 +55,7 @@ typedef enum {
 typedef enum {
   PM_ORDER_DEFAULT = -1,  /* REDBLACK for every solver */
   PM_ORDER_REFERENCE = 0, /* the reference's in-place lexicographic order, run as an exact
-                             hyperplane wavefront: bit-identical to the reference */
+                             pipeline of tiles: bit-identical to the reference */
   PM_ORDER_JACOBI = 1,    /* ping-pong: every neighbour from the previous iterate
                              (diverges for solver 1, whose pressure update uses the
                              pre-update velocities; solvers 2 and 3 are stable) */
@@ -287,9 +287,12 @@ typedef struct {
                                head is admitted (0 = 64; negative = strict first come,
                                first served).  A request larger than the whole budget
                                completes at once with PM_ERR_NOMEM. */
-  int relaunch_sweeps;      /* mixed form: 0 (default) runs a round's FP32 sweeps as one
-                               persistent kernel walking a device tile queue; 1 launches
-                               every sweep separately (same results bit for bit) */
+  int relaunch_sweeps;      /* mixed form: 0 (default) runs a round's FP32 sweeps as
+                               overlapped launches over packed records (for samples
+                               these do not hold, and for a launch shape set by the
+                               caller, as one persistent kernel walking a device tile
+                               queue); 1 launches every sweep separately (same results
+                               bit for bit) */
 } pm_server_config;
 
 typedef struct pm_server pm_server;
@@ -327,8 +330,9 @@ pm_status pm_server_request_bytes(pm_server* s, const pm_params* p, size_t* byte
  * of the device queue; cut smaller when the resident set is small), shape[1]
  * CTAs per SM and shape[2] threads per block of the mixed form's persistent
  * round, shape[3] threads per block of the other batched kernels.  With
- * cfg.autotune the server picks them per size class of the resident set; the
- * getter reports the current choice.  The setter pins a shape (autotuning
+ * cfg.autotune the server picks them per size class of the resident set where
+ * a round uses them (not the mixed form's overlapped sweeps over packed
+ * records); the getter reports the current choice.  The setter pins a shape (autotuning
  * stops; 128 threads with 1-8 CTAs or 256 with 1-4, threads 128 / 256 / 512)
  * from the next round on; call it between rounds.  Every shape gives the same
  * results bit for bit.  No counterpart in the reference. */

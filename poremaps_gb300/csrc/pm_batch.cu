@@ -7,8 +7,8 @@
 // same device function as the single-problem kernels (pm_stencil.cuh), so a
 // sample's fields are identical whether it is solved alone or in a batch.
 // The mixed form's correction and residual are the compact store of
-// pm_compact.cu (one float4 per fluid-list position), as the single-problem
-// kernel 8 uses them.
+// pm_compact.cu (one float4 per fluid-list position), as in the single-problem
+// kernels 8 to 13.
 #include <stddef.h>
 
 #include <algorithm>
