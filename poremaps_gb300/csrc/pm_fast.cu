@@ -44,7 +44,7 @@ cudaError_t sweep64_exact(Fields<double> A, Fields<double> B, const uint8_t* cod
 // 128 registers, so that all of a voxel's loads are in flight at once; three
 // leave 80, no spills, and keep the pipe busier where there is enough work:
 // Jacobi on the 128^3 pack 44.0 us against 46.5 with two, red-black 57.6 against
-// 59.8; a 97x61x118 pack 25.7 against 21.9 (its half-sweeps are 1.2 waves of
+// 59.8 (55.7 with the hint of update64); a 97x61x118 pack 25.7 against 21.9 (its half-sweeps are 1.2 waves of
 // three).  With the whole stencil loaded and plain launches: 48.4, 63 and 26.1.
 template <int SOLVER, int PHASE, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_sweep64_pf(Fields<double> A, Fields<double> B,

@@ -371,6 +371,18 @@ struct Own64 {
   double u, v, w, p;
 };
 
+// A load whose line may be the first to leave L2 (first), or a plain one.
+__device__ __forceinline__ double ld_last(const double* p, bool first) {
+  unsigned long long go, stay;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(go));
+  asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(stay));
+  double v;
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;"
+               : "=d"(v)
+               : "l"(p), "l"(first ? go : stay));
+  return v;
+}
+
 template <int SOLVER, int PHASE, int LD, int P3 = 1>
 __device__ __forceinline__ void update64(const Fields<double>& A, const Fields<double>& B,
                                          long long c, int x, int y, int z, const Grid& g, int code,
@@ -404,10 +416,18 @@ __device__ __forceinline__ void update64(const Fields<double>& A, const Fields<d
   const long long ay = first(cy, ym, yp), by = second(cy, sy, yp);
   const long long az = first(cz, zm, zp), bz = second(cz, sz, zp);
   const double *U = A.u + c, *V = A.v + c, *W = A.w + c, *Q = A.p + c;
-  o.u = ldA(U, LD);
-  o.v = ldA(V, LD);
-  o.w = ldA(W, LD);
-  o.p = (P3 != 0 && z == g.NZ - 3) ? (P3 == 1 ? 3.0 : 0.0) : ldA(Q, LD);
+  // the black pass's own values: the last use of the old state's lines (but for
+  // second neighbours), which make room for the new state, all of it read by
+  // the next sweep.  Where L2 holds one state and not both (128^3 pack): 57.7 ->
+  // 55.7 us; where it holds both (97x61x118, 112^3) as before; where it does not
+  // hold one, without the hint (160^3 98 against 96 us, 224^3 217 against 203).
+  // The same hint on a Jacobi sweep's reads of the plane below: 44.1 -> 45.1.
+  const bool one_fits = g.pl64 * g.NZ <= (128ll << 20) / 32;
+  auto own = [&](const double* q) { return PHASE == 2 ? ld_last(q, one_fits) : ldA(q, LD); };
+  o.u = own(U);
+  o.v = own(V);
+  o.w = own(W);
+  o.p = (P3 != 0 && z == g.NZ - 3) ? (P3 == 1 ? 3.0 : 0.0) : own(Q);
   const double uxp = ldA(U + xp, LD), vyp = ldA(V + yp, LD), wzp = ldA(W + zp, LD);
   const bool lx = left_solid(cx), ly = left_solid(cy), lz = left_solid(cz);
   const double P = -Relax64<SOLVER>::Dt * o.p;
