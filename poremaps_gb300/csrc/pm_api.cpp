@@ -456,6 +456,10 @@ pm_status choose_correction_kernel(pm_problem* pr, int kernel) {
       pr->crec = pr->crec_own ? pr->crec_own : (uint4*)pr->cslot4;
       CK(compact_records(pr->cmeta, pr->cslot4, pr->cslot2, pr->nlist, pr->crec, pr->cslot2,
                          pr->st));
+      // the first sweep may follow directly, and it reads records before it
+      // waits for the launch before it (ld_record)
+      pm_status s = device_sync(pr, "packed records");
+      if (s != PM_OK) return s;
     }
     if (k == 0 || k == 3)
       CK(zmarch_create(&pr->zp, pr->g, pr->E[0], pr->E[1], pr->R, pr->codes, 0, k == 3));

@@ -161,7 +161,8 @@ pm_status iterate_n(pm_problem* pr, int n);
 // device memory kept for the next problems (free for any allocation of theirs)
 size_t pool_bytes();
 // packs the compact store's slots into records in their place (kernel 13),
-// where they hold the medium's offsets
+// where they hold the medium's offsets; before a correction sweep comes the
+// residual of the problem's first iteration, a plain launch (ld_record)
 pm_status problem_pack(pm_problem* pr);
 // mixed form: fold the FP32 correction into the FP64 state (no-op otherwise)
 pm_status problem_flush(pm_problem* pr);

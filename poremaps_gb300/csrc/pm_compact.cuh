@@ -314,7 +314,9 @@ __device__ __forceinline__ float4 ld_stream(const float4* p) {
   return v;
 }
 
-// (set up long before any sweep: the read-only path)
+// Overlapped sweeps load records before they wait for the launch before them:
+// between the packing and such a sweep on its stream there has to be a
+// synchronisation or a plain launch.  Then the read-only path is safe too.
 __device__ __forceinline__ uint4 ld_record(const uint4* p) {
   uint4 v;
   asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"

@@ -1,0 +1,125 @@
+"""The host runtime (problem set-up, kernel choice, device memory, the server's
+rounds) on a stand-in for the device (fake_device.cpp): what reaches the device
+in which order, with which buffers, and how much memory is held.  No GPU."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import poremaps_gb300 as pm
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "poremaps_gb300", "csrc")
+CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+GB = 1 << 30
+
+
+@pytest.fixture(scope="session")
+def built(tmp_path_factory):
+    cxx = shutil.which("g++")
+    if not cxx or not os.path.exists(os.path.join(CUDA_INC, "cuda_runtime.h")):
+        pytest.skip("g++ or the CUDA headers are missing")
+    so = str(tmp_path_factory.mktemp("host") / "libhost.so")
+    subprocess.run([cxx, "-O1", "-g", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic",
+                    "-I", CUDA_INC,
+                    os.path.join(HERE, "fake_device.cpp"), os.path.join(CSRC, "pm_api.cpp"),
+                    os.path.join(CSRC, "pm_server.cpp"), "-lpthread", "-o", so], check=True)
+    return so
+
+
+class Host:
+    """The library over the stand-in; a copy of its own for each test, since the
+    kernel choices and kept blocks live as long as the library."""
+
+    def __init__(self, so):
+        L = self.L = C.CDLL(so)
+        P, vp = C.POINTER, C.c_void_p
+        L.pm_last_error.restype = C.c_char_p
+        L.fake_trace.restype = C.c_char_p
+        L.fake_used.restype = C.c_size_t
+        L.fake_set_cost.argtypes = [C.c_char_p, C.c_double]
+        L.fake_set_memory.argtypes = [C.c_int, C.c_size_t]
+        L.pm_problem_create.argtypes = [P(pm.Params), vp, P(vp)]
+        for f in ("pm_problem_destroy", "pm_server_destroy"):
+            getattr(L, f).argtypes = [vp]
+        L.pm_iterate.argtypes = [vp, C.c_int]
+        L.pm_get_kernel.argtypes = [vp, P(C.c_int)]
+        L.pm_problem_footprint.argtypes = [P(pm.Params), P(C.c_size_t)]
+        L.pm_server_create.argtypes = [P(pm.ServerConfig), P(vp)]
+        L.pm_server_submit.argtypes = [vp, P(pm.Params), vp, P(C.c_uint64)]
+        L.pm_server_step.argtypes = [vp, P(C.c_int)]
+        L.pm_server_poll.argtypes = [vp, P(pm.Completion), C.c_int, P(C.c_int)]
+        L.pm_server_cancel.argtypes = [vp, C.c_uint64]
+
+    def trace(self):
+        t = self.L.fake_trace().decode().split("\n")
+        self.L.fake_reset_trace()
+        return t
+
+    def params(self, shape, **kw):
+        p = pm.Params()
+        assert self.L.pm_params_default(C.byref(p)) == 0
+        p.size[0], p.size[1], p.size[2] = shape
+        for k, v in kw.items():
+            setattr(p, k, v)
+        return p
+
+    def create(self, shape, fluid, **kw):
+        """(status, handle); shape (nx, ny, nz), `fluid` fluid voxels."""
+        p = self.params(shape, **kw)
+        self.L.fake_set_fluid(fluid)
+        geom = np.zeros(min(p.size[0] * p.size[1] * p.size[2], 1 << 20), np.uint8)
+        h = C.c_void_p()
+        return self.L.pm_problem_create(C.byref(p), geom.ctypes.data, C.byref(h)), h
+
+    def kernel(self, h):
+        k = C.c_int()
+        assert self.L.pm_get_kernel(h, C.byref(k)) == 0
+        return k.value
+
+
+@pytest.fixture
+def host(built, tmp_path):
+    return Host(shutil.copy(built, tmp_path / "lib.so"))
+
+
+def bad(trace):
+    return [t for t in trace if t.startswith(("null", "unordered"))]
+
+
+# ------------------------------------------------------------------ launch order
+@pytest.mark.parametrize("kw", [dict(precision=1), dict(precision=1, kernel=13),
+                                dict(order=pm.ORDER_JACOBI), dict(order=pm.ORDER_REDBLACK)])
+def test_overlapped_sweeps_follow_their_set_up_data(host, kw):
+    """Overlapped sweeps read records and list entries before they wait for the
+    launch before them: what wrote these has to be ordered before that launch.
+    Twice: the second problem finds the kernel choice made."""
+    for _ in range(2):
+        st, h = host.create((40, 40, 40), 20000, **kw)
+        assert st == 0, host.L.pm_last_error()
+        assert host.L.pm_iterate(h, 5) == 0
+        t = host.trace()
+        assert any(n in t for n in ("dc_inner_cr", "sweep64"))
+        assert bad(t) == []
+        host.L.pm_problem_destroy(h)
+
+
+@pytest.mark.parametrize("it_eval", [1, 2, 10])
+def test_server_sweeps_follow_their_set_up_data(host, it_eval):
+    cfg = pm.ServerConfig(0, 0, 1, 0, 0, 0, 0)
+    s = C.c_void_p()
+    assert host.L.pm_server_create(C.byref(cfg), C.byref(s)) == 0
+    host.L.fake_set_fluid(5000)
+    geom = np.zeros(24 ** 3, np.uint8)
+    p = host.params((24, 24, 24), it_eval=it_eval, max_iter=34)
+    t = C.c_uint64()
+    for _ in range(3):
+        assert host.L.pm_server_submit(s, C.byref(p), geom.ctypes.data, C.byref(t)) == 0
+    active = C.c_int(1)
+    while active.value:
+        assert host.L.pm_server_step(s, C.byref(active)) == 0, host.L.pm_last_error()
+    assert bad(host.trace()) == []
+    host.L.pm_server_destroy(s)
