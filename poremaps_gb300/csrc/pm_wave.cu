@@ -8,7 +8,7 @@
 // grouped in tiles of kTileY x kTileZ; at its step t a tile updates the voxel
 // x = t - ly - lz of each of its columns, so a -1 / -2 neighbour inside the
 // tile was updated one / two steps before, and its values lie in a ring of
-// shared memory.  Tiles take tickets in lexicographic order and wait only for
+// shared memory.  Tiles take tickets in the order of pm_wave.h and wait only for
 // values of the tiles below them in y and z, whose tickets are smaller and so
 // running or done: no co-residency is needed.  Those values are handed over in
 // an exchange copy of the fields, filled with kEmpty before the sweep: a tile
@@ -39,6 +39,7 @@
 
 #include "pm_internal.h"
 #include "pm_stencil.cuh"
+#include "pm_wave.h"
 
 namespace pm {
 
@@ -141,17 +142,18 @@ __device__ __forceinline__ double velocity_lane(double c, double visc, double pm
 template <int SOLVER>
 __global__ void __launch_bounds__(kWaveThreads)
     k_wave(Fields<double> f, Fields<double> X, const uint8_t* codes, Grid g, int tiles_y,
-           int* ticket, int* err, int polls) {
+           int tiles_z, int* ticket, int* err, int polls) {
   __shared__ double ring[4][kSlot];
   __shared__ double tab[8][4];
   __shared__ unsigned short cases[256];
-  __shared__ int sh_ticket;
+  __shared__ int sh_tile[2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) sh_ticket = atomicAdd(ticket, 1) + 1;
+  if (threadIdx.x == 0)
+    wave_tile(atomicAdd(ticket, 1) + 1, tiles_y, tiles_z, sh_tile[0], sh_tile[1]);
   fill_tables(tab, cases);
   for (int i = threadIdx.x; i < 4 * kSlot; i += blockDim.x) (&ring[0][0])[i] = 0.0;
   __syncthreads();
-  const int tile = sh_ticket, tY = tile % tiles_y, tZ = tile / tiles_y;
+  const int tY = sh_tile[0], tZ = sh_tile[1];
   const int y0 = tY * kTileY, z0 = tZ * kTileZ;
   const int ncy = min(kTileY, g.ny - y0), ncz = min(kTileZ, g.nz - z0);
   const int t_last = g.nx - 1 + ncy - 1 + ncz - 1;
@@ -426,7 +428,7 @@ cudaError_t launch_wave(Fields<double> f, const uint8_t* codes, const Grid& g, i
   double* b = exchange + kXoff64;
   const Fields<double> X = {b, b + g.alloc64, b + 2 * g.alloc64, b + 3 * g.alloc64};
   auto* k = solver == 1 ? k_wave<1> : solver == 2 ? k_wave<2> : k_wave<3>;
-  k<<<ty * tz, kWaveThreads, 0, st>>>(f, X, codes, g, ty, (int*)exchange, err,
+  k<<<ty * tz, kWaveThreads, 0, st>>>(f, X, codes, g, ty, tz, (int*)exchange, err,
                                       g_wave_fail.load() ? 1 : kWavePolls);
   count_launches(1);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;

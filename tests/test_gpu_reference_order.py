@@ -27,6 +27,20 @@ def test_sweep_tiles(nx, ny, nz, bc, solver):
                 assert np.array_equal(a, b)
 
 
+# more tiles than are resident at once, with few voxels in x each
+@pytest.mark.parametrize("nx,ny,nz,bc", [(1, 121, 130, 0), (2, 30, 601, 1), (3, 601, 30, 4)])
+def test_sweep_many_thin_tiles(nx, ny, nz, bc):
+    g = synth.random_solid((nz, ny, nx), 0.3, nx)
+    orc = OracleProblem(g, bc, 2)
+    orc.iterate(7, "reference")
+    with pm.Problem(g, None, boundary_method=bc, order="reference") as pr:
+        pr.iterate(7)
+        got = pr.fields()
+    f = orc.fields()
+    for a, b in zip(got, (f.u, f.v, f.w, f.p)):
+        assert np.array_equal(a, b)
+
+
 def test_sweep_wait_runs_out():
     """With the test hook a tile gives up after its first look at a neighbour's
     values: the sweep ends, the call reports it, and the problem sweeps on."""
