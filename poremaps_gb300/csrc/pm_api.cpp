@@ -397,7 +397,8 @@ void release_unused_store(pm_problem* pr) {
 }
 
 // Tuned correction-sweep choices: (kernel, brick order of the fluid list) per
-// (size, solver, boundary method, porosity bucket).  The choice depends on the
+// (size, solver, boundary method, porosity bucket, whether the packed records
+// hold the medium, which decides the candidates).  The choice depends on the
 // medium's size, porosity and boundary family, not on its exact pattern, and
 // every candidate gives bitwise identical fields: problems alike (e.g. the
 // rotated runs of one tensor) share one tuning, and concurrent tunings are
@@ -406,13 +407,14 @@ struct Cand {
   int k, b[3];
   int var = 0;  // kernel 13: launch variant (launch_dc_inner_cr)
 };
-using TuneKey = std::array<long long, 6>;
+using TuneKey = std::array<long long, 7>;
 std::mutex g_tune_mu;
 std::map<TuneKey, Cand> g_tuned;
 
 TuneKey tune_key(const pm_problem* pr) {
   return {pr->g.nx, pr->g.ny, pr->g.nz, pr->solver, pr->prm.boundary_method,
-          (long long)llround(20.0 * (double)pr->nlist / (double)pr->g.nvox)};
+          (long long)llround(20.0 * (double)pr->nlist / (double)pr->g.nvox),
+          compact_records_fit(pr->g, pr->nlist)};
 }
 
 // The kernel a problem will use if it is already known (pinned, the packed
@@ -436,6 +438,8 @@ pm_status choose_correction_kernel(pm_problem* pr, int kernel) {
     if (pr->bp) { brick_destroy(pr->bp); pr->bp = nullptr; }
     pr->kern = k;
     const bool cpt = k >= 8 && k <= 13;
+    if (!(cpt ? pr->c_base : pr->f32_base))
+      return set_error(PM_ERR_INVALID, "the correction store of kernel %d is not allocated", k);
     if (cpt) b = kLex;
     // the list is rebuilt only when its order changes (creation builds it
     // lexicographic), and the compact store is set up once per list order

@@ -123,3 +123,21 @@ def test_server_sweeps_follow_their_set_up_data(host, it_eval):
         assert host.L.pm_server_step(s, C.byref(active)) == 0, host.L.pm_last_error()
     assert bad(host.trace()) == []
     host.L.pm_server_destroy(s)
+
+
+# ------------------------------------------------------------------ kernel choice
+def test_choices_of_media_that_records_hold_and_do_not_hold(host):
+    """Two media of one size and porosity on either side of the records' limit of
+    2^27 - 1 fluid voxels: each gets the kernel chosen among its own candidates,
+    over a store that exists, whichever comes first."""
+    fits, not_fits, shape = (1 << 27) - 2, 1 << 27, (640, 640, 640)
+    host.L.fake_set_cost(b"dc_inner_pf", 0.1)  # a kernel over the padded store wins
+    seen = []
+    for fluid in (not_fits, fits, not_fits, fits):
+        st, h = host.create(shape, fluid, precision=1)
+        assert st == 0, host.L.pm_last_error()
+        assert host.L.pm_iterate(h, 3) == 0
+        seen.append(host.kernel(h))
+        assert bad(host.trace()) == []
+        host.L.pm_problem_destroy(h)
+    assert seen == [6, 13, 6, 13]
