@@ -154,8 +154,13 @@ static std::mutex g_pin_mu;
 static std::vector<double*> g_pin_free;
 
 size_t pool_bytes() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  return g_pool_bytes;
+  size_t n = 0;
+  for (auto& b : g_pool)
+    if (b.dev == dev) n += b.bytes;
+  return n;
 }
 
 static cudaError_t pinned_slot(double** out) {

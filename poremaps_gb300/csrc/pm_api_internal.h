@@ -158,7 +158,8 @@ long long problem_nvox(const pm_problem* pr);
 cudaStream_t problem_stream(const pm_problem* pr);
 // calc_flow pieces shared with the server
 pm_status iterate_n(pm_problem* pr, int n);
-// device memory kept for the next problems (free for any allocation of theirs)
+// memory of the current device kept for the next problems (free for any
+// allocation of theirs)
 size_t pool_bytes();
 // packs the compact store's slots into records in their place (kernel 13),
 // where they hold the medium's offsets; before a correction sweep comes the

@@ -141,3 +141,53 @@ def test_choices_of_media_that_records_hold_and_do_not_hold(host):
         assert bad(host.trace()) == []
         host.L.pm_problem_destroy(h)
     assert seen == [6, 13, 6, 13]
+
+
+# ------------------------------------------------------------------ device memory
+def test_kept_blocks_of_another_device_are_not_free_here(host):
+    """What destroyed problems left on another device does not count as free
+    memory of this one."""
+    L = host.L
+    L.fake_set_memory(0, 200 << 20)
+    L.pm_set_device(1)
+    st, h = host.create((96, 96, 96), 400000, order=pm.ORDER_JACOBI)
+    assert st == 0
+    L.pm_problem_destroy(h)
+    assert L.fake_used(1) > 60 << 20  # kept
+    L.pm_set_device(0)
+    host.trace()
+    st, _ = host.create((150, 150, 150), 1000, order=pm.ORDER_JACOBI)  # 250 MB
+    assert st == pm.PM_ERR_NOMEM
+    assert b"needs" in L.pm_last_error() and "out of memory" not in host.trace()
+    L.pm_set_device(1)  # there they do
+    L.fake_set_memory(1, L.fake_used(1) + (2 << 20))
+    st, h = host.create((96, 96, 96), 400000, order=pm.ORDER_JACOBI)
+    assert st == 0, L.pm_last_error()
+    L.pm_problem_destroy(h)
+
+
+def test_server_budget_leaves_out_kept_blocks_of_another_device(host):
+    L = host.L
+    L.pm_set_device(1)
+    st, h = host.create((160, 160, 160), 400000, order=pm.ORDER_JACOBI)
+    assert st == 0
+    L.pm_problem_destroy(h)
+    L.pm_set_device(0)
+    p = host.params((96, 96, 96), it_eval=10, max_iter=34, precision=0)
+    need = C.c_size_t()
+    assert L.pm_problem_footprint(C.byref(p), C.byref(need)) == 0
+    L.fake_set_memory(0, int(1.7 * need.value))  # 0.8 of it holds one, not two
+    L.fake_set_fluid(400000)
+    cfg = pm.ServerConfig(0, 0, 0, 0, 0, 0, 0)
+    s, t = C.c_void_p(), C.c_uint64()
+    assert L.pm_server_create(C.byref(cfg), C.byref(s)) == 0
+    geom = np.zeros(96 ** 3, np.uint8)
+    for _ in range(2):
+        assert L.pm_server_submit(s, C.byref(p), geom.ctypes.data, C.byref(t)) == 0
+    active = C.c_int(1)
+    while active.value:
+        assert L.pm_server_step(s, C.byref(active)) == 0, L.pm_last_error()
+    done, n = (pm.Completion * 2)(), C.c_int()
+    assert L.pm_server_poll(s, done, 2, C.byref(n)) == 0
+    assert n.value == 2 and [c.status for c in done] == [0, 0]
+    L.pm_server_destroy(s)
