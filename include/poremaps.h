@@ -213,6 +213,11 @@ pm_status pm_solve_tensor(const pm_params* p, const uint8_t* geom, double K[9],
 /* ---- device selection, timing and re-use (bench and serving support) ---- */
 /* Select the CUDA device for problems created afterwards by this thread. */
 pm_status pm_set_device(int device);
+/* Device memory of destroyed problems (at most 1 GB) is kept for the next ones;
+ * this gives it back to the device, for other users of it in the process or
+ * beside it.  Memory in use stays.  May be called at any time, from any thread.
+ * No counterpart in the reference. */
+pm_status pm_release_memory(void);
 /* Back to the initial state (iteration 0, fields as after pm_problem_create). */
 pm_status pm_problem_reset(pm_problem* pr);
 /* n iterations, then (if check) the convergence evaluation of

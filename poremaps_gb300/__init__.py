@@ -85,7 +85,7 @@ EXPORTS = ["pm_last_error", "pm_last_error_copy", "pm_version", "pm_params_defau
            "pm_iterate", "pm_compute_convergence", "pm_compute_permeability", "pm_get_porosity",
            "pm_get_iteration", "pm_get_fields", "pm_set_fields", "pm_resume_outputs",
            "pm_get_neighborhood", "pm_write_outputs",
-           "pm_run_inp", "pm_solve_tensor", "pm_set_device", "pm_problem_reset",
+           "pm_run_inp", "pm_solve_tensor", "pm_set_device", "pm_release_memory", "pm_problem_reset",
            "pm_block_timed", "pm_block_group_timed", "pm_kernel_time", "pm_kernel_launches", "pm_get_kernel", "pm_get_brick", "pm_reduce_fields_noalloc",
            "pm_server_create", "pm_server_destroy",
            "pm_server_submit", "pm_server_step", "pm_server_poll", "pm_server_stats",
@@ -130,6 +130,7 @@ def load_library(path: str = LIB_PATH):
         "pm_run_inp": (C.c_int, [C.c_char_p, P(Params), P(Result)]),
         "pm_solve_tensor": (C.c_int, [P(Params), vp, P(C.c_double), P(Result)]),
         "pm_set_device": (C.c_int, [C.c_int]),
+        "pm_release_memory": (C.c_int, []),
         "pm_problem_reset": (C.c_int, [vp]),
         "pm_block_timed": (C.c_int, [vp, C.c_int, C.c_int, P(C.c_double), P(C.c_double),
                                      P(C.c_double)]),
@@ -351,6 +352,12 @@ class Problem:
 
 def set_device(device: int) -> None:
     _check(load_library().pm_set_device(device))
+
+
+def release_memory() -> None:
+    """pm_release_memory: device memory kept from closed problems (at most 1 GB)
+    goes back to the device, e.g. for PyTorch's allocator."""
+    _check(load_library().pm_release_memory())
 
 
 def block_group_timed(problems, n: int, check: bool = True, permeability=None):

@@ -54,9 +54,10 @@ std::atomic<int> g_fail_alloc{0};
 // makes and destroys its problems (the tensor's three rotations, the server's
 // samples) spends 0.2 to 2 ms a problem in cudaMalloc and cudaFree otherwise
 // (the tensor of a 128^3 pack: 27.9 -> 26.9 ms, 24 server samples 63 -> 59 ms).
-// At most kPoolBytes are kept; they count as free memory, and an
-// allocation that fails gives them back to the device and is tried again.  A
-// block is put here only once no work uses it.
+// At most kPoolBytes are kept; they count as free memory, an allocation of this
+// library that fails gives them back to the device and is tried again, and
+// pm_release_memory gives them back to others.  A block is put here only once
+// no work uses it.
 constexpr size_t kPoolBytes = 1ull << 30;
 struct PoolBlock {
   void* p;
@@ -68,10 +69,31 @@ std::vector<PoolBlock> g_pool;
 std::map<void*, PoolBlock> g_pool_out;  // every block dev_alloc handed out
 size_t g_pool_bytes = 0;
 
-void pool_give_back() {  // g_pool_mu held
+bool pool_give_back() {  // g_pool_mu held; whether there was any
+  const bool any = !g_pool.empty();
   for (auto& b : g_pool) cudaFree(b.p);
   g_pool.clear();
   g_pool_bytes = 0;
+  return any;
+}
+
+bool pool_release() {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  return pool_give_back();
+}
+
+cudaError_t cuda_alloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !pool_release()) return e;
+  cudaGetLastError();
+  return cudaMalloc(p, bytes);
+}
+
+cudaError_t cuda_alloc_async(void** p, size_t bytes, cudaStream_t st) {
+  cudaError_t e = cudaMallocAsync(p, bytes, st);
+  if (e != cudaErrorMemoryAllocation || !pool_release()) return e;
+  cudaGetLastError();
+  return cudaMallocAsync(p, bytes, st);
 }
 
 template <typename T>
@@ -99,9 +121,8 @@ cudaError_t dev_alloc(T** ptr, size_t bytes) {
     g_pool.erase(g_pool.begin() + best);
   } else {
     e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && !g_pool.empty()) {
+    if (e == cudaErrorMemoryAllocation && pool_give_back()) {
       cudaGetLastError();
-      pool_give_back();
       e = cudaMalloc(&p, bytes);
     }
     if (e != cudaSuccess) return e;
@@ -1172,6 +1193,11 @@ pm_status pm_solve(pm_problem* pr, pm_result* res) {
 
 pm_status pm_set_device(int device) {
   CK(cudaSetDevice(device));
+  return PM_OK;
+}
+
+pm_status pm_release_memory(void) {
+  pool_release();
   return PM_OK;
 }
 

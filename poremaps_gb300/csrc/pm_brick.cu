@@ -194,7 +194,7 @@ cudaError_t brick_create(BrickPlan** out, const Grid& g, float4* E0, float4* E1,
   const long long nb = (long long)nbx * nby * nbz;
   std::vector<int> start((size_t)nb);
   int* d_start = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d_start, sizeof(int) * (size_t)nb, st);
+  cudaError_t e = cuda_alloc_async((void**)&d_start, sizeof(int) * (size_t)nb, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_start, 0xff, sizeof(int) * (size_t)nb, st);
   if (e == cudaSuccess && nlist > 0) {
     k_brick_starts<<<(nlist + 255) / 256, 256, 0, st>>>(list, nlist, g, bx, by, bz, nbx, nby,
@@ -220,10 +220,10 @@ cudaError_t brick_create(BrickPlan** out, const Grid& g, float4* E0, float4* E1,
   }
   pl->nwork = (int)work.size();
   work.push_back(make_int4(0, 0, 0, nlist));  // end of the last brick's range
-  e = cudaMalloc((void**)&pl->work, sizeof(int4) * work.size());
+  e = cuda_alloc((void**)&pl->work, sizeof(int4) * work.size());
   if (e == cudaSuccess)
     e = cudaMemcpy(pl->work, work.data(), sizeof(int4) * work.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&pl->err, sizeof(int));
+  if (e == cudaSuccess) e = cuda_alloc((void**)&pl->err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(pl->err, 0, sizeof(int));
   if (e != cudaSuccess) {
     brick_destroy(pl);

@@ -71,6 +71,12 @@ void count_launches(int n);
 int sm_count();
 unsigned long long launches_total();
 
+// cudaMalloc and cudaMallocAsync for whatever is not a problem's own buffer:
+// where they fail, the device blocks kept for later problems (pm_api.cpp) are
+// given back and they are tried again.
+cudaError_t cuda_alloc(void** p, size_t bytes);
+cudaError_t cuda_alloc_async(void** p, size_t bytes, cudaStream_t st);
+
 // ---------------------------------------------------------------- launchers
 // All launchers are asynchronous on `st` and return the launch error.
 cudaError_t launch_codes(const uint8_t* raw, uint8_t* codes, const Grid& g, cudaStream_t st);

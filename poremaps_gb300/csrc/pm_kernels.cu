@@ -268,7 +268,7 @@ cudaError_t launch_fluid_list(const uint8_t* codes, const Grid& g, int* list, in
   const long long nseg = (long long)b.nbx * b.nby * b.nbz * b.by * b.bz;
   if (nseg > (1LL << 30)) return cudaErrorInvalidValue;
   int* tmp = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&tmp, sizeof(int) * 2 * (size_t)nseg, st);
+  cudaError_t e = cuda_alloc_async((void**)&tmp, sizeof(int) * 2 * (size_t)nseg, st);
   if (e != cudaSuccess) return e;
   k_seg_counts<<<(unsigned)nseg, 128, 0, st>>>(codes, g, b, parity, tmp);
   k_scan_rows<<<1, 1024, 0, st>>>(tmp, (int)nseg, tmp + nseg, count);

@@ -125,7 +125,7 @@ pm_status grow(T** d, size_t* cap, size_t n) {
   size_t c = std::max(n, *cap * 2 + 16);
   if (*d) cudaFree(*d);
   *d = nullptr;
-  SCK(cudaMalloc((void**)d, c * sizeof(T)));
+  SCK(cuda_alloc((void**)d, c * sizeof(T)));
   *cap = c;
   return PM_OK;
 }
@@ -347,7 +347,7 @@ pm_status upload(pm_server* s) {
     s->d_part = nullptr;
     s->h_part = nullptr;
     size_t c = s->h_items.size() * 2 + 16;
-    SCK(cudaMalloc((void**)&s->d_part, c * sizeof(double)));
+    SCK(cuda_alloc((void**)&s->d_part, c * sizeof(double)));
     SCK(cudaMallocHost((void**)&s->h_part, c * sizeof(double)));
     s->cap_part = c;
   }

@@ -290,7 +290,7 @@ cudaError_t zmarch_create(ZmarchPlan** out, const Grid& g, float4* E0, float4* E
     delete pl;
     return cudaErrorInvalidValue;
   }
-  cudaError_t e = cudaMalloc((void**)&pl->err, sizeof(int));
+  cudaError_t e = cuda_alloc((void**)&pl->err, sizeof(int));
   if (e != cudaSuccess) {
     delete pl;
     return e;

@@ -104,6 +104,7 @@ int fake_pending() {
 
 // ---- CUDA runtime
 cudaError_t cudaMalloc(void** p, size_t n) { return device_alloc(p, n); }
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return device_alloc(p, n); }
 cudaError_t cudaFree(void* p) {  // waits for the device, as the real one
   if (!p) return cudaSuccess;
   for (auto* s : g_streams) settle(s);

@@ -49,3 +49,18 @@ def test_blocks_of_several_threads():
     for t in ts:
         t.join()
     assert not bad
+
+
+def test_release_memory():
+    """Given back while a problem runs, and used again afterwards."""
+    want = [solve((18, 20, 22), i, i) for i in range(len(KINDS))]
+    g = synth.random_solid((18, 20, 22), 0.3, 0)
+    with pm.Problem(g, None, boundary_method=0, **KINDS[0]) as p:
+        p.iterate(11)
+        pm.release_memory()
+        got = [solve((18, 20, 22), i, i) for i in range(len(KINDS))]
+        pm.release_memory()
+        p.iterate(12)
+        assert all(np.array_equal(a, b) for a, b in zip(p.fields(), want[0]))
+    for a, b in zip(got, want):
+        assert all(np.array_equal(x, y) for x, y in zip(a, b))

@@ -191,3 +191,52 @@ def test_server_budget_leaves_out_kept_blocks_of_another_device(host):
     assert L.pm_server_poll(s, done, 2, C.byref(n)) == 0
     assert n.value == 2 and [c.status for c in done] == [0, 0]
     L.pm_server_destroy(s)
+
+
+def test_kept_blocks_are_bounded_and_given_back(host):
+    """At most 1 GB is kept, the oldest blocks leave first, and
+    pm_release_memory gives everything back."""
+    L = host.L
+    for n in (128, 150, 170, 190, 210, 256):
+        hs = []
+        for _ in range(3):
+            st, h = host.create((n, n, n), 1000, order=pm.ORDER_JACOBI)
+            assert st == 0, L.pm_last_error()
+            hs.append(h)
+        for h in hs:
+            L.pm_problem_destroy(h)
+        assert 0 < L.fake_used(0) <= GB
+    assert L.pm_release_memory() == 0
+    assert L.fake_used(0) == 0
+    st, h = host.create((40, 40, 40), 1000, order=pm.ORDER_JACOBI)
+    assert st == 0 and L.pm_release_memory() == 0 and L.fake_used(0) > 0  # in use: stays
+    assert L.pm_iterate(h, 3) == 0
+    L.pm_problem_destroy(h)
+
+
+@pytest.mark.parametrize("left", [0, 1 << 12])
+def test_any_allocation_gets_what_is_kept(host, left):
+    """Not only a problem's own buffers: where the server's tables do not fit
+    beside the kept blocks, these are given back."""
+    L = host.L
+    cfg = pm.ServerConfig(GB, 0, 1, 0, 0, 0, 0)
+    s, t = C.c_void_p(), C.c_uint64()
+    assert L.pm_server_create(C.byref(cfg), C.byref(s)) == 0
+    st, other = host.create((128, 128, 128), 1000, order=pm.ORDER_JACOBI)
+    assert st == 0
+    p = host.params((64, 64, 64), it_eval=10, max_iter=34, precision=1)
+    L.fake_set_fluid(100000)
+    geom = np.zeros(64 ** 3, np.uint8)
+    st, h = host.create((64, 64, 64), 100000, precision=1, kernel=8, order=pm.ORDER_JACOBI)
+    assert st == 0  # its blocks are what the request will use
+    L.pm_problem_destroy(other)
+    L.pm_problem_destroy(h)
+    L.fake_set_memory(0, L.fake_used(0) + left)
+    assert L.pm_server_submit(s, C.byref(p), geom.ctypes.data, C.byref(t)) == 0
+    active = C.c_int(1)
+    while active.value:
+        assert L.pm_server_step(s, C.byref(active)) == 0, L.pm_last_error()
+    done, n = (pm.Completion * 1)(), C.c_int()
+    assert L.pm_server_poll(s, done, 1, C.byref(n)) == 0
+    assert n.value == 1 and done[0].status == 0
+    L.pm_server_destroy(s)
