@@ -733,13 +733,18 @@ pm_status pm_server_submit(pm_server* s, const pm_params* p, const uint8_t* geom
 pm_status pm_server_step(pm_server* s, int* active) {
   if (!s) return set_error(PM_ERR_INVALID, "bad arguments");
   std::lock_guard<std::mutex> lk(s->mu);
-  pm_status e;
-  if ((e = admit(s)) != PM_OK) return e;
-  if (!s->res.empty()) {
-    if (s->dirty && (e = rebuild(s)) != PM_OK) return e;
-    if ((e = run_block(s)) != PM_OK) return e;
-    if ((e = after_block(s)) != PM_OK) return e;
-    if ((e = admit(s)) != PM_OK) return e;
+  pm_status e = admit(s);
+  if (e == PM_OK && !s->res.empty()) {
+    if (s->dirty) e = rebuild(s);
+    if (e == PM_OK) e = run_block(s);
+    if (e == PM_OK) e = after_block(s);
+    if (e == PM_OK) e = admit(s);
+  }
+  if (e != PM_OK) {
+    // part of a round may have been launched: between steps no work uses the
+    // samples' memory (dev_free gives it to the next problem without a wait)
+    cudaStreamSynchronize(s->st);
+    return e;
   }
   if (active) *active = (int)(s->res.size() + s->queue.size());
   return PM_OK;

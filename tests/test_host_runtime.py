@@ -240,3 +240,25 @@ def test_any_allocation_gets_what_is_kept(host, left):
     assert L.pm_server_poll(s, done, 1, C.byref(n)) == 0
     assert n.value == 1 and done[0].status == 0
     L.pm_server_destroy(s)
+
+
+@pytest.mark.parametrize("nth", [1, 2, 5])
+def test_failed_round_leaves_no_work_on_memory_that_is_kept(host, nth):
+    """A launch that fails in the middle of a round: what was launched before it
+    has ended when the call returns, so a cancelled sample's memory, which the
+    next problem takes at once, is not in use."""
+    L = host.L
+    cfg = pm.ServerConfig(0, 0, 1, 0, 0, 0, 0)  # no graphs: launched one by one
+    s, t = C.c_void_p(), C.c_uint64()
+    assert L.pm_server_create(C.byref(cfg), C.byref(s)) == 0
+    L.fake_set_fluid(5000)
+    geom = np.zeros(24 ** 3, np.uint8)
+    p = host.params((24, 24, 24), it_eval=10, max_iter=104)
+    assert L.pm_server_submit(s, C.byref(p), geom.ctypes.data, C.byref(t)) == 0
+    active = C.c_int()
+    assert L.pm_server_step(s, C.byref(active)) == 0
+    L.fake_fail_launch(nth)
+    assert L.pm_server_step(s, C.byref(active)) == 3
+    assert L.fake_pending() == 0
+    assert L.pm_server_cancel(s, t) == 0
+    L.pm_server_destroy(s)
