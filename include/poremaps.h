@@ -364,6 +364,12 @@ pm_status pm_debug_round_wait(unsigned extra, int polls);
  * the sweep's caller gets PM_ERR_CUDA with the device still usable.  0 turns
  * it off.  Process-wide. */
 pm_status pm_debug_tma_fail(int on);
+/* Problems made from now on sweep in the given launch form instead of the one
+ * their timings pick, so a test can compare forms that lose on its machine:
+ * fp64_form 0 one voxel per thread, 1 / 2 one wave of 2 / 3 CTAs per SM, 3 one
+ * wave of 2 with the whole stencil loaded; record_variant 0 / 1 / 2 CTAs of
+ * 256 / 512 / 1024 threads of kernel 13; -1 restores.  Process-wide. */
+pm_status pm_debug_launch_forms(int fp64_form, int record_variant);
 
 #ifdef __cplusplus
 }

@@ -91,7 +91,7 @@ EXPORTS = ["pm_last_error", "pm_last_error_copy", "pm_version", "pm_params_defau
            "pm_server_submit", "pm_server_step", "pm_server_poll", "pm_server_stats",
            "pm_server_clock_ms", "pm_server_cancel", "pm_debug_fail_alloc",
            "pm_problem_footprint", "pm_server_request_bytes", "pm_debug_round_wait",
-           "pm_debug_tma_fail", "pm_server_launch_shape", "pm_server_set_launch_shape"]
+           "pm_debug_tma_fail", "pm_debug_launch_forms", "pm_server_launch_shape", "pm_server_set_launch_shape"]
 
 _lib = None
 
@@ -153,6 +153,7 @@ def load_library(path: str = LIB_PATH):
         "pm_debug_fail_alloc": (C.c_int, [C.c_int]),
         "pm_debug_round_wait": (C.c_int, [C.c_uint, C.c_int]),
         "pm_debug_tma_fail": (C.c_int, [C.c_int]),
+        "pm_debug_launch_forms": (C.c_int, [C.c_int, C.c_int]),
         "pm_problem_footprint": (C.c_int, [P(Params), P(C.c_size_t)]),
         "pm_server_request_bytes": (C.c_int, [vp, P(Params), P(C.c_size_t)]),
         "pm_server_launch_shape": (C.c_int, [vp, P(C.c_int)]),
@@ -193,6 +194,12 @@ def debug_round_wait(extra: int, polls: int) -> None:
 def debug_tma_fail(on: bool) -> None:
     """pm_debug_tma_fail: z-march launches report a timed-out first wait."""
     _check(load_library().pm_debug_tma_fail(int(bool(on))))
+
+
+def debug_launch_forms(fp64_form: int = -1, record_variant: int = -1) -> None:
+    """pm_debug_launch_forms: problems made from now on sweep in these launch
+    forms (-1: the ones their timings pick)."""
+    _check(load_library().pm_debug_launch_forms(int(fp64_form), int(record_variant)))
 
 
 def _check(st: int):

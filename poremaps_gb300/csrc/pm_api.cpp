@@ -50,6 +50,9 @@ pm_status set_error(pm_status st, const char* fmt, ...) {
 // fails as cudaMalloc does when the device is out of memory.
 std::atomic<int> g_fail_alloc{0};
 
+// pm_debug_launch_forms: the form problems made from now on take, -1 their own.
+std::atomic<int> g_force_form64{-1}, g_force_variant{-1};
+
 // Device blocks of destroyed problems, kept for the next ones: a call that
 // makes and destroys its problems (the tensor's three rotations, the server's
 // samples) spends 0.2 to 2 ms a problem in cudaMalloc and cudaFree otherwise
@@ -330,13 +333,23 @@ pm_status iterate64(pm_problem* pr) {
   return PM_OK;
 }
 
-// Launch form of each FP64 phase (persistent with 2 or 3 CTAs per SM, or one
-// voxel per thread), timed on the problem: the lists' lengths decide how evenly
-// the waves of each form end (a 97x61x118 pack sweeps in 21.9 us with 2 CTAs
-// per SM and 25.7 with 3, a 128^3 one in 59.8 and 57.6).  All give identical
-// fields; the trials sweep the two states, which are set up again afterwards.
+// Launch form of each FP64 phase (kForm64*), timed on the problem.  The whole
+// stencil is kept unless another form is 1 % faster: it is, where the voxels are
+// dense or their states exceed L2 (Jacobi of a 256^3 medium of porosity 0.6 538 us
+// against 549 with the reduced loads, 512^3 4,253 against 4,346, red-black of
+// 400^3 2,081 against 2,141), the reduced loads where they are not (red-black of
+// a 48^3 medium 8.2 us against 11.4, of a 256^3 one of porosity 0.2 252 against
+// 285), and the lists' lengths decide how evenly the waves of 2 and 3 end (a
+// 97x61x118 pack sweeps in 21.9 us with 2 and 25.7 with 3, a 128^3 one in 59.8
+// and 57.6).
+// All give identical fields; the trials sweep the two states, which are set up
+// again afterwards.
 pm_status choose_fp64_shapes(pm_problem* pr) {
   if (pr->exact) return PM_OK;
+  if (const int forced = g_force_form64.load(); forced >= 0) {
+    for (int& f : pr->pf64) f = forced;
+    return PM_OK;
+  }
   static std::mutex mu;
   static std::map<std::array<long long, 7>, std::array<int, 3>> tuned;
   std::lock_guard<std::mutex> lock(mu);
@@ -348,13 +361,18 @@ pm_status choose_fp64_shapes(pm_problem* pr) {
     for (int i = 0; i < 3; ++i) pr->pf64[i] = hit->second[i];
     return PM_OK;
   }
-  // whole iterations in turn between the two states, as a solve runs them
+  // whole iterations in turn between the two states, as a solve runs them; a
+  // second trial where they are short, and one voxel per thread only there (its
+  // gain is that it fills the device evenly)
+  constexpr float kLong = 1.0f;  // ms of a trial
   auto set = [&](int form) { for (int& f : pr->pf64) f = form; };
-  float t[3] = {1e30f, 1e30f, 1e30f};
-  for (int form = 2; form >= 0; --form) {
+  float t[kForms64];
+  for (int form = kForms64 - 1; form >= 0; --form) {
+    t[form] = 1e30f;
+    if (form == kForm64One && t[kForm64Whole] >= kLong) break;
     set(form);
     pm_status s = iterate64(pr);
-    for (int trial = 0; trial < 2 && s == PM_OK; ++trial) {
+    for (int trial = 0; trial < 2 && s == PM_OK && !(trial && t[form] >= kLong); ++trial) {
       CK(cudaEventRecord(pr->ev0, pr->st));
       for (int r = 0; r < 4 && s == PM_OK; ++r) s = iterate64(pr);
       CK(cudaEventRecord(pr->ev1, pr->st));
@@ -365,8 +383,10 @@ pm_status choose_fp64_shapes(pm_problem* pr) {
     }
     if (s != PM_OK) return s;
   }
-  const int pf = t[2] < t[1] ? 2 : 1;
-  set(t[0] < 0.98f * t[pf] ? 0 : pf);
+  int best = kForm64Whole;
+  for (int form = 0; form < kForm64Whole; ++form)
+    if (t[form] < 0.99f * t[kForm64Whole] && t[form] < t[best]) best = form;
+  set(best);
   pr->cur = 0;
   CK(launch_init64(pr->F[0], pr->codes, pr->g, pr->st));
   CK(launch_copy_fields64(pr->F[1], pr->F[0], pr->g, pr->st));
@@ -869,6 +889,14 @@ pm_status pm_debug_fail_alloc(int nth) {
   return PM_OK;
 }
 
+pm_status pm_debug_launch_forms(int fp64_form, int record_variant) {
+  if (fp64_form < -1 || fp64_form >= kForms64 || record_variant < -1 || record_variant > 2)
+    return set_error(PM_ERR_INVALID, "forms: FP64 -1..%d, records -1..2", kForms64 - 1);
+  g_force_form64.store(fp64_form);
+  g_force_variant.store(record_variant);
+  return PM_OK;
+}
+
 pm_status pm_params_default(pm_params* p) {
   if (!p) return set_error(PM_ERR_INVALID, "params is NULL");
   memset(p, 0, sizeof(*p));
@@ -1049,6 +1077,7 @@ pm_status pm::problem_create(const pm_params* p, const uint8_t* geom, int rot_ax
     }
     pm_status ts = choose_correction_kernel(pr, p->kernel);
     if (ts != PM_OK) return fail(ts);
+    if (const int forced = g_force_variant.load(); forced >= 0) pr->cvar = forced;
   }
   if (pr->precision == PM_PREC_FP64 && pr->order != PM_ORDER_REFERENCE) {
     pm_status ts = choose_fp64_shapes(pr);

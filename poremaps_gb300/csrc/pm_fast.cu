@@ -42,7 +42,7 @@ cudaError_t sweep64_exact(Fields<double> A, Fields<double> B, const uint8_t* cod
 // pack) and, between a warp's instructions there, its loads; the half-sweeps
 // of that pack also miss L2 (their two states touch 120 MB).  Two CTAs leave
 // 128 registers, so that all of a voxel's loads are in flight at once; three
-// leave 80, no spills, and keep the pipe busier where there is enough work:
+// leave 80, next to no spills, and keep the pipe busier where there is enough work:
 // Jacobi on the 128^3 pack 44.0 us against 46.5 with two, red-black 57.6 against
 // 59.8 (55.7 with the hint of update64); a 97x61x118 pack 25.7 against 21.9 (its half-sweeps are 1.2 waves of
 // three).  With the whole stencil loaded and plain launches: 48.4, 63 and 26.1.
@@ -66,6 +66,30 @@ __global__ void __launch_bounds__(256, MINB) k_sweep64_pf(Fields<double> A, Fiel
   }
 }
 
+// The whole stencil per voxel, two CTAs per SM (128 registers), plain launches:
+// no load waits for the code byte.  Bound as the sweep above; where its voxels'
+// values come from beyond L2, or are dense, the 37 loads cost less than the wait
+// (choose_fp64_shapes has both sides), and beside other problems the plain
+// launches do (a CTA that waits for its predecessor takes the place of one that
+// could run).
+template <int SOLVER, int PHASE>
+__global__ void __launch_bounds__(256, 2) k_sweep64_whole(Fields<double> A, Fields<double> B,
+                                                         const uint8_t* codes, const int* list,
+                                                         int nlist, Grid g) {
+  __shared__ double centre[16];
+  fill_centre64<SOLVER>(centre);
+  __syncthreads();
+  const int stride = gridDim.x * blockDim.x;
+  int q = blockIdx.x * blockDim.x + threadIdx.x;
+  int lin = q < nlist ? __ldg(list + q) : 0;
+  for (; q < nlist; q += stride) {
+    const int qn = q + stride;
+    const int next = qn < nlist ? __ldg(list + qn) : 0;
+    sweep64_voxel<SOLVER, PHASE, false>(A, B, codes, g, lin, nullptr, centre);
+    lin = next;
+  }
+}
+
 template <int SOLVER, int MINB>
 static cudaError_t sweep_pf(Fields<double> A, Fields<double> B, const uint8_t* codes,
                             const int* list, int nlist, const Grid& g, int phase,
@@ -80,13 +104,18 @@ static cudaError_t sweep_pf(Fields<double> A, Fields<double> B, const uint8_t* c
 template <int SOLVER>
 static cudaError_t sweep_fast_s(Fields<double> A, Fields<double> B, const uint8_t* codes,
                                 const int* list, int nlist, const Grid& g, int phase,
-                                int persistent, cudaStream_t st) {
+                                int form, cudaStream_t st) {
   const int blocks = (nlist + 255) / 256;
   if (blocks < 1) return cudaSuccess;
-  if (persistent == 1) {
+  if (form == kForm64Two) {
     return sweep_pf<SOLVER, 2>(A, B, codes, list, nlist, g, phase, st);
-  } else if (persistent == 2) {
+  } else if (form == kForm64Three) {
     return sweep_pf<SOLVER, 3>(A, B, codes, list, nlist, g, phase, st);
+  } else if (form == kForm64Whole) {
+    const int wave = std::min(blocks, 2 * sm_count());
+    auto* k = phase == 0 ? k_sweep64_whole<SOLVER, 0>
+                         : phase == 1 ? k_sweep64_whole<SOLVER, 1> : k_sweep64_whole<SOLVER, 2>;
+    k<<<wave, 256, 0, st>>>(A, B, codes, list, nlist, g);
   } else {
     if (phase == 0) k_sweep64_fast<SOLVER, 0><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
     else if (phase == 1) k_sweep64_fast<SOLVER, 1><<<blocks, 256, 0, st>>>(A, B, codes, list, nlist, g);
@@ -98,11 +127,11 @@ static cudaError_t sweep_fast_s(Fields<double> A, Fields<double> B, const uint8_
 
 cudaError_t launch_sweep64(Fields<double> A, Fields<double> B, const uint8_t* codes,
                            const int* list, int nlist, const Grid& g, int solver, int exact,
-                           int phase, cudaStream_t st, int persistent) {
+                           int phase, cudaStream_t st, int form) {
   if (exact) return sweep64_exact(A, B, codes, list, nlist, g, solver, phase, st);
-  if (solver == 1) return sweep_fast_s<1>(A, B, codes, list, nlist, g, phase, persistent, st);
-  if (solver == 2) return sweep_fast_s<2>(A, B, codes, list, nlist, g, phase, persistent, st);
-  return sweep_fast_s<3>(A, B, codes, list, nlist, g, phase, persistent, st);
+  if (solver == 1) return sweep_fast_s<1>(A, B, codes, list, nlist, g, phase, form, st);
+  if (solver == 2) return sweep_fast_s<2>(A, B, codes, list, nlist, g, phase, form, st);
+  return sweep_fast_s<3>(A, B, codes, list, nlist, g, phase, form, st);
 }
 
 // ------------------------------------------------------------------ mixed precision

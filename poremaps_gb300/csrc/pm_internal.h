@@ -108,11 +108,13 @@ void wave_debug_fail(int on);
 
 // Ping-pong Jacobi (phase 0) and red (1) / black (2) half-sweeps from A into B
 // over the fluid list; periodic halo copies and the pressure reapply fused.
-// persistent: 1, 2: one wave of 2 / 3 CTAs per SM walking the list (0: one voxel
-// per thread); all give identical fields.
+// form (fast arithmetic): one voxel per thread; one wave of 2 / 3 CTAs per SM
+// walking the list, launches overlapping; one wave of 2 with the whole stencil
+// loaded and plain launches.  All give identical fields.
+enum { kForm64One = 0, kForm64Two = 1, kForm64Three = 2, kForm64Whole = 3, kForms64 = 4 };
 cudaError_t launch_sweep64(Fields<double> A, Fields<double> B, const uint8_t* codes,
                            const int* list, int nlist, const Grid& g, int solver, int exact,
-                           int phase, cudaStream_t st, int persistent = 1);
+                           int phase, cudaStream_t st, int form = kForm64Two);
 
 // Mixed precision (defect correction).  x: FP64 state, e: FP32 correction
 // (ping-pong), r: FP32 residual; e and r interleaved (float4 u, v, w, p).

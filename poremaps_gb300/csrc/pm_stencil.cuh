@@ -197,14 +197,21 @@ __device__ __forceinline__ double centre64(int g1, int g2) {
 
 // Off-centre coefficients of a wall stencil of case cs times K' (see case_coef).
 template <int SOLVER>
-__device__ __forceinline__ double2 case_coef64(int cs) {
+__device__ __forceinline__ void case_coef64(int cs, double& cA, double& cB) {
   constexpr double K = Relax64<SOLVER>::K;
   switch (cs) {
-    case 1: return make_double2(0.0, 0.0);
-    case 2: case 3: return make_double2(K * (8.0 / 3.0), 0.0);
-    case 4: case 5: return make_double2(K * 2.0, K * -0.2);
-    default: return make_double2(K, K);
+    case 1: cA = 0.0; cB = 0.0; break;
+    case 2: case 3: cA = K * (8.0 / 3.0); cB = 0.0; break;
+    case 4: case 5: cA = K * 2.0; cB = K * -0.2; break;
+    default: cA = K; cB = K; break;
   }
+}
+
+template <int SOLVER>
+__device__ __forceinline__ double2 case_coef64(int cs) {
+  double2 k;
+  case_coef64<SOLVER>(cs, k.x, k.y);
+  return k;
 }
 
 // A block's shared tables: centre coefficients by the two case groups,
@@ -216,9 +223,14 @@ struct Tables64 {
 };
 
 template <int SOLVER>
+__device__ __forceinline__ void fill_centre64(double* centre) {
+  for (int i = threadIdx.x; i < 16; i += blockDim.x) centre[i] = centre64<SOLVER>(i >> 2, i & 3);
+}
+
+template <int SOLVER>
 __device__ __forceinline__ void fill_tables64(Tables64& t) {
+  fill_centre64<SOLVER>(t.centre);
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    if (i < 16) t.centre[i] = centre64<SOLVER>(i >> 2, i & 3);
     if (i < 8) t.coef[i] = case_coef64<SOLVER>(i);
     int cx, cy, cz;
     decode_cases(i >= 1 && i <= 216 ? i : 216, cx, cy, cz);
@@ -442,6 +454,57 @@ __device__ __forceinline__ void update64(const Fields<double>& A, const Fields<d
   pn = fma(-kC2 * kDt, dv, o.p);
 }
 
+// The same update from the whole stencil (update64 loads only what the cases
+// use, so its addresses wait for the code byte; here the 37 loads do not).
+// centre: the block's table of centre coefficients; the others from selects on
+// the cases.
+template <int SOLVER>
+__device__ __forceinline__ double vel64_whole(double c, double am, double ap, int cs1, double ll1,
+                                              double l1, double r1, double rr1, int cs2,
+                                              double ll2, double l2, double r2, double rr2,
+                                              double pm, double P, bool lsolid,
+                                              const double* centre) {
+  double cA1, cB1, cA2, cB2, A1, B1, A2, B2;
+  case_coef64<SOLVER>(cs1, cA1, cB1);
+  case_coef64<SOLVER>(cs2, cA2, cB2);
+  case_pick<double>(cs1, ll1, l1, r1, rr1, A1, B1);
+  case_pick<double>(cs2, ll2, l2, r2, rr2, A2, B2);
+  constexpr double K = Relax64<SOLVER>::K;
+  const double Cc = centre[case_group(cs1) * 4 + case_group(cs2)];
+  double t = lsolid ? 0.0 : fma(Relax64<SOLVER>::Dt, pm, P);
+  t = fma(Cc, c, t);
+  t = fma(K, am, t);
+  t = fma(K, ap, t);
+  t = fma(cA1, A1, t);
+  t = fma(cB1, B1, t);
+  t = fma(cA2, A2, t);
+  t = fma(cB2, B2, t);
+  return (SOLVER != 3 && lsolid) ? 0.0 : t;
+}
+
+template <int SOLVER, int PHASE>
+__device__ __forceinline__ void update64_whole(const Fields<double>& A, const Fields<double>& B,
+                                               long long c, int x, int y, int z, const Grid& g,
+                                               int code, const double* centre, double& un,
+                                               double& vn, double& wn, double& pn) {
+  Stencil<double> s;
+  gather<double, PHASE>(s, A, B, c, x, y, z, g, g.px64, g.pl64);
+  int cx, cy, cz;
+  decode_cases(code, cx, cy, cz);
+  const bool lx = left_solid(cx), ly = left_solid(cy), lz = left_solid(cz);
+  const double P = -Relax64<SOLVER>::Dt * s.pc;
+  double d0 = 0.0;
+  if (SOLVER == 1) d0 = ((s.wzp - s.wc) + (s.vyp - s.vc)) + (s.uxp - s.uc);
+  un = vel64_whole<SOLVER>(s.uc, s.uxm, s.uxp, cy, s.uymm, s.uym, s.uyp, s.uypp, cz, s.uzmm,
+                           s.uzm, s.uzp, s.uzpp, s.pxm, P, lx, centre);
+  vn = vel64_whole<SOLVER>(s.vc, s.vym, s.vyp, cx, s.vxmm, s.vxm, s.vxp, s.vxpp, cz, s.vzmm,
+                           s.vzm, s.vzp, s.vzpp, s.pym, P, ly, centre);
+  wn = vel64_whole<SOLVER>(s.wc, s.wzm, s.wzp, cx, s.wxmm, s.wxm, s.wxp, s.wxpp, cy, s.wymm,
+                           s.wym, s.wyp, s.wypp, s.pzm, P, lz, centre);
+  const double dv = SOLVER == 1 ? d0 : ((s.wzp - wn) + (s.vyp - vn)) + (s.uxp - un);
+  pn = fma(-kC2 * kDt, dv, s.pc);
+}
+
 // Write the new values of interior voxel (x, y, z) and, on periodic axes,
 // its halo copies (the halo exchange fused into the sweep).  The pressure
 // reapply is fused too: the z-halo copies on planes 1 and NZ-2 hold nz+2 and 2
@@ -495,10 +558,12 @@ __device__ __forceinline__ void lin_to_xyz(int lin, const Grid& g, int& x, int& 
 }
 
 // One voxel of an FP64 sweep (Jacobi phase 0, red 1, black 2) from A into B.
+// whole: the table of centre coefficients, for update64_whole.
 template <int SOLVER, int PHASE, bool EXACT, int LD = kLdNc>
 __device__ __forceinline__ void sweep64_voxel(const Fields<double>& A, const Fields<double>& B,
                                               const uint8_t* codes, const Grid& g, int lin,
-                                              const Tables64* tab = nullptr) {
+                                              const Tables64* tab = nullptr,
+                                              const double* whole = nullptr) {
   int x, y, z;
   lin_to_xyz(lin, g, x, y, z);
   if (PHASE && (((x + y + z) & 1) != PHASE - 1)) return;  // (x+y+z) - 6 has the same parity
@@ -510,6 +575,8 @@ __device__ __forceinline__ void sweep64_voxel(const Fields<double>& A, const Fie
     Stencil<double> s;
     gather<double, PHASE, LD>(s, A, B, c, x, y, z, g, px, pl);
     update_exact<SOLVER>(s, code, un, vn, wn, pn);
+  } else if (whole) {
+    update64_whole<SOLVER, PHASE>(A, B, c, x, y, z, g, code, whole, un, vn, wn, pn);
   } else {
     Own64 o;
     update64<SOLVER, PHASE, LD>(A, B, c, x, y, z, g, code, tab, o, un, vn, wn, pn);

@@ -268,7 +268,11 @@ cudaError_t launch_wave(Fields<double> f, const uint8_t*, const Grid&, int, doub
 void wave_debug_fail(int) {}
 cudaError_t launch_sweep64(Fields<double> A, Fields<double> B, const uint8_t*, const int* list,
                            int, const Grid&, int, int exact, int, cudaStream_t st, int form) {
-  return launch("sweep64", st, exact || form == 0 ? kPlain : kOverlapped, {A.u, B.u, list});
+  const std::string cost = "sweep64 form " + std::to_string(form);
+  note(cost);
+  g_cost["sweep64"] = g_cost.count(cost) ? g_cost[cost] : 1.0;
+  const bool plain = exact || form == kForm64One || form == kForm64Whole;
+  return launch("sweep64", st, plain ? kPlain : kOverlapped, {A.u, B.u, list});
 }
 cudaError_t launch_dc_correct_list(Fields<double> x, const float4* e, const int* list, int,
                                    const Grid&, cudaStream_t st) {

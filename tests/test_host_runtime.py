@@ -143,6 +143,28 @@ def test_choices_of_media_that_records_hold_and_do_not_hold(host):
     assert seen == [6, 13, 6, 13]
 
 
+def forms(trace):
+    return [int(t.split()[-1]) for t in trace if t.startswith("sweep64 form")]
+
+
+@pytest.mark.parametrize("costs,want", [((1.0, 1.0, 1.0, 1.0), 3), ((1.0, 0.995, 0.992, 1.0), 3),
+                                        ((1.0, 0.97, 0.98, 1.0), 1), ((1.0, 0.97, 0.96, 1.0), 2),
+                                        ((0.9, 0.97, 0.96, 1.0), 0)])
+@pytest.mark.parametrize("scale", [0.01, 1.0])
+def test_fp64_form_is_timed(host, costs, want, scale):
+    """The whole-stencil form unless another is at least 1 % faster; sweeps that
+    take long are timed with fewer of them, and not one voxel per thread."""
+    for i, c in enumerate(costs):
+        host.L.fake_set_cost(b"sweep64 form %d" % i, c * scale)
+    st, h = host.create((40, 40, 40), 20000, order=pm.ORDER_JACOBI)
+    assert st == 0
+    assert len(forms(host.trace())) <= (36 if scale < 0.1 else 15)
+    assert host.L.pm_iterate(h, 2) == 0
+    if scale == 1.0 and want == 0:
+        want = 2
+    assert forms(host.trace()) == [want, want]
+
+
 # ------------------------------------------------------------------ device memory
 def test_kept_blocks_of_another_device_are_not_free_here(host):
     """What destroyed problems left on another device does not count as free
