@@ -183,13 +183,17 @@ __global__ void __launch_bounds__(kChunk, MINB)
 }
 
 // r = F(x) - x in FP64 from the padded state (as dc_residual_voxel), stored
-// at the list position, and e1 = r.
+// at the list position, and e1 = r.  The whole stencil, as k_sweep64_whole:
+// nothing overlaps a residual's launch, and with the loads reduced to what the
+// cases use, the wait for the code byte shows (128^3 medium of porosity 0.6 94.2 us
+// against 96.4, 256^3 of 0.2 227.1 against 231.6; over the padded store 94.3
+// against 99.9 and 227.7 against 237.1).
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 2) k_dc_residual_c(Fields<double> X, float4* R,
                                                         float4* E, const uint8_t* codes,
                                                         const int* list, int nlist, Grid g) {
-  __shared__ Tables64 tab;
-  fill_tables64<SOLVER>(tab);
+  __shared__ double centre[16];
+  fill_centre64<SOLVER>(centre);
   __syncthreads();
   const int stride = gridDim.x * blockDim.x;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -197,7 +201,7 @@ __global__ void __launch_bounds__(256, 2) k_dc_residual_c(Fields<double> X, floa
   for (; q < nlist; q += stride) {
     const int qn = q + stride;
     const int next = qn < nlist ? __ldg(list + qn) : 0;
-    residual_c_voxel<SOLVER>(X, R, E, codes, g, q, lin, &tab);
+    residual_c_voxel<SOLVER>(X, R, E, codes, g, q, lin, centre);
     lin = next;
   }
 }

@@ -358,18 +358,20 @@ __device__ __forceinline__ void inner_c_voxel(const float4* __restrict__ E,
 }
 
 // r = F(x) - x in FP64 from the padded state (as dc_residual_voxel), stored
-// at list position q, and e1 = r.
+// at list position q, and e1 = r.  centre: the block's table, for the whole
+// stencil (null: reduced loads).
 template <int SOLVER>
 __device__ __forceinline__ void residual_c_voxel(const Fields<double>& X, float4* R, float4* E,
                                                  const uint8_t* codes, const Grid& g, int q,
-                                                 int lin, const Tables64* tab = nullptr) {
+                                                 int lin, const double* centre = nullptr) {
   int x, y, z;
   lin_to_xyz(lin, g, x, y, z);
   const int code = codes[((long long)z * g.NY + y) * g.pxc + x];
   const long long c = (long long)z * g.pl64 + (long long)y * g.px64 + x;
   Own64 o;
   double un, vn, wn, pn;
-  update64<SOLVER, 0, kLdNc>(X, X, c, x, y, z, g, code, tab, o, un, vn, wn, pn);
+  if (centre) update64_whole<SOLVER, 0>(X, X, c, x, y, z, g, code, centre, o, un, vn, wn, pn);
+  else update64<SOLVER, 0, kLdNc>(X, X, c, x, y, z, g, code, nullptr, o, un, vn, wn, pn);
   const double pstored = (z == g.NZ - 3) ? __ldg(X.p + c) : o.p;
   const float4 rv = make_float4((float)(un - o.u), (float)(vn - o.v), (float)(wn - o.w),
                                 (float)(pn - pstored));

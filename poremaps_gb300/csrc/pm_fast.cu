@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(256, 2) k_dc_residual(Fields<double> X, float4
                                                       const uint8_t* codes, const int* list,
                                                       int nlist, Grid g) {
   // persistent, next list entry prefetched (as the FP64 sweeps)
-  __shared__ Tables64 tab;
-  fill_tables64<SOLVER>(tab);
+  __shared__ double centre[16];
+  fill_centre64<SOLVER>(centre);
   __syncthreads();
   const int stride = gridDim.x * blockDim.x;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256, 2) k_dc_residual(Fields<double> X, float4
   for (; q < nlist; q += stride) {
     const int qn = q + stride;
     const int next = qn < nlist ? __ldg(list + qn) : 0;
-    dc_residual_voxel<SOLVER>(X, R, E, codes, g, lin, &tab);
+    dc_residual_voxel<SOLVER>(X, R, E, codes, g, lin, centre);
     lin = next;
   }
 }

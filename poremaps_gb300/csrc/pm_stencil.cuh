@@ -485,10 +485,11 @@ __device__ __forceinline__ double vel64_whole(double c, double am, double ap, in
 template <int SOLVER, int PHASE>
 __device__ __forceinline__ void update64_whole(const Fields<double>& A, const Fields<double>& B,
                                                long long c, int x, int y, int z, const Grid& g,
-                                               int code, const double* centre, double& un,
-                                               double& vn, double& wn, double& pn) {
+                                               int code, const double* centre, Own64& o,
+                                               double& un, double& vn, double& wn, double& pn) {
   Stencil<double> s;
   gather<double, PHASE>(s, A, B, c, x, y, z, g, g.px64, g.pl64);
+  o = {s.uc, s.vc, s.wc, s.pc};
   int cx, cy, cz;
   decode_cases(code, cx, cy, cz);
   const bool lx = left_solid(cx), ly = left_solid(cy), lz = left_solid(cz);
@@ -576,7 +577,8 @@ __device__ __forceinline__ void sweep64_voxel(const Fields<double>& A, const Fie
     gather<double, PHASE, LD>(s, A, B, c, x, y, z, g, px, pl);
     update_exact<SOLVER>(s, code, un, vn, wn, pn);
   } else if (whole) {
-    update64_whole<SOLVER, PHASE>(A, B, c, x, y, z, g, code, whole, un, vn, wn, pn);
+    Own64 o;
+    update64_whole<SOLVER, PHASE>(A, B, c, x, y, z, g, code, whole, o, un, vn, wn, pn);
   } else {
     Own64 o;
     update64<SOLVER, PHASE, LD>(A, B, c, x, y, z, g, code, tab, o, un, vn, wn, pn);
@@ -638,14 +640,14 @@ __device__ __forceinline__ void write_voxel4(float4* B, long long c, int x, int 
 template <int SOLVER>
 __device__ __forceinline__ void dc_residual_voxel(const Fields<double>& X, float4* R, float4* E,
                                                   const uint8_t* codes, const Grid& g, int lin,
-                                                  const Tables64* tab = nullptr) {
+                                                  const double* centre) {
   int x, y, z;
   lin_to_xyz(lin, g, x, y, z);
   int code = codes[((long long)z * g.NY + y) * g.pxc + x];
   long long c = (long long)z * g.pl64 + (long long)y * g.px64 + x;
   Own64 o;
   double un, vn, wn, pn;
-  update64<SOLVER, 0, kLdNc>(X, X, c, x, y, z, g, code, tab, o, un, vn, wn, pn);
+  update64_whole<SOLVER, 0>(X, X, c, x, y, z, g, code, centre, o, un, vn, wn, pn);
   const double pstored = (z == g.NZ - 3) ? __ldg(X.p + c) : o.p;
   float ru = (float)(un - o.u), rv = (float)(vn - o.v), rw = (float)(wn - o.w),
         rp = (float)(pn - pstored);
