@@ -317,20 +317,43 @@ pm_status correction_sweep(pm_problem* pr, int src) {
   return PM_OK;
 }
 
-// One iteration of the FP64 forms: sweep A -> B (fused exchange + reapply), swap.
-pm_status iterate64(pm_problem* pr) {
-  Fields<double> A = pr->F[pr->cur], B = pr->F[1 - pr->cur];
+// Launch form of an FP64 phase over n voxels: the one that won alone
+// (choose_fp64_shapes), or, for problems that share the device, what suits
+// them all.  Where their states exceed L2, the whole stencil in plain launches:
+// overlapped CTAs that wait take the place of other problems' CTAs, and the
+// reduced loads gain little there (three 128^3 packs, red-black: 151 us against
+// 167 with 2 CTAs per SM and 156 with 3; three 96^3 media 100, 115, 104; a tensor
+// of a 128^3 pack 157 against 170).  Within L2, 3 CTAs per SM once the problems'
+// blocks no longer fit beside each other (three 48^3 media, Jacobi: 12 us
+// against 14 whole and 15.5 with 2; 56^3 red-black 19, 22.5, 24.6), else as alone.
+int form64(const pm_problem* pr, int phase, int n) {
+  if (pr->share <= 1 || pr->pf64_forced) return pr->pf64[phase];
+  const size_t states = (size_t)pr->share * 2 * 4 * sizeof(double) * (size_t)pr->g.alloc64;
+  if (states > kL2Bytes) return kForm64Whole;
+  return (long long)pr->share * ((n + 255) / 256) > 3LL * sm_count() ? kForm64Three
+                                                                     : pr->pf64[phase];
+}
+
+// An iteration's sweeps A -> B (fused exchange + reapply) of the FP64 forms.
+pm_status sweeps64(pm_problem* pr, Fields<double> A, Fields<double> B) {
+  auto sweep = [&](int phase, const int* list, int n) {
+    return launch_sweep64(A, B, pr->codes, list, n, pr->g, pr->solver, pr->exact, phase, pr->st,
+                          form64(pr, phase, n));
+  };
   if (pr->order == PM_ORDER_JACOBI) {
-    CK(launch_sweep64(A, B, pr->codes, pr->list, pr->nlist, pr->g, pr->solver, pr->exact, 0,
-                      pr->st, pr->pf64[0]));
+    CK(sweep(0, pr->list, pr->nlist));
   } else {
-    CK(launch_sweep64(A, B, pr->codes, pr->list, pr->nred, pr->g, pr->solver, pr->exact, 1,
-                      pr->st, pr->pf64[1]));
-    CK(launch_sweep64(A, B, pr->codes, pr->list + pr->nred, pr->nlist - pr->nred, pr->g,
-                      pr->solver, pr->exact, 2, pr->st, pr->pf64[2]));
+    CK(sweep(1, pr->list, pr->nred));
+    CK(sweep(2, pr->list + pr->nred, pr->nlist - pr->nred));
   }
-  pr->cur = 1 - pr->cur;
   return PM_OK;
+}
+
+// One iteration of the FP64 forms: sweep, swap.
+pm_status iterate64(pm_problem* pr) {
+  pm_status s = sweeps64(pr, pr->F[pr->cur], pr->F[1 - pr->cur]);
+  pr->cur = 1 - pr->cur;
+  return s;
 }
 
 // Launch form of each FP64 phase (kForm64*), timed on the problem.  The whole
@@ -348,6 +371,7 @@ pm_status choose_fp64_shapes(pm_problem* pr) {
   if (pr->exact) return PM_OK;
   if (const int forced = g_force_form64.load(); forced >= 0) {
     for (int& f : pr->pf64) f = forced;
+    pr->pf64_forced = true;
     return PM_OK;
   }
   static std::mutex mu;
@@ -679,7 +703,7 @@ pm_status pm::iterate_n(pm_problem* pr, int n) {
   const int phase = pr->precision == PM_PREC_MIXED ? pr->iteration % pr->mixed_inner : 0;
   for (const auto& b : pr->graphs) {
     if (b.n == n && b.cur == pr->cur && b.ecur == pr->ecur && b.dc_pos == pr->dc_pos &&
-        b.phase == phase) {
+        b.phase == phase && b.share == pr->share) {
       CK(cudaGraphLaunch(b.exec, pr->st));
       count_launches(b.launches);
       pr->cur = b.cur1;
@@ -692,6 +716,7 @@ pm_status pm::iterate_n(pm_problem* pr, int n) {
   }
   pm_problem::BlockGraph b;
   b.n = n; b.cur = pr->cur; b.ecur = pr->ecur; b.dc_pos = pr->dc_pos; b.phase = phase;
+  b.share = pr->share;
   const unsigned long long l0 = launches_total();
   CK(cudaStreamBeginCapture(pr->st, cudaStreamCaptureModeThreadLocal));
   pm_status s = iterate_direct(pr, n);
@@ -1258,6 +1283,16 @@ pm_status pm_block_group_timed(pm_problem** prs, int count, int n, int check,
   for (int i = 0; i < count; ++i)
     if (!prs[i]) return set_error(PM_ERR_INVALID, "bad arguments");
   pm_problem* lead = prs[0];
+  // the sweeps of the group share the device until it is joined
+  struct Share {
+    pm_problem** prs;
+    int count;
+    Share(pm_problem** p, int n) : prs(p), count(n) { set(n); }
+    ~Share() { set(1); }
+    void set(int n) {
+      for (int i = 0; i < count; ++i) prs[i]->share = n;
+    }
+  } share(prs, count);
   // fork: every stream starts after the start event on the first stream
   CK(cudaEventRecord(lead->ev0, lead->st));
   for (int i = 1; i < count; ++i) CK(cudaStreamWaitEvent(prs[i]->st, lead->ev0, 0));
@@ -1307,16 +1342,8 @@ pm_status pm_kernel_time(pm_problem* pr, int kernel, int n, double* avg_ms) {
         if (s != PM_OK) return s;
       }
     } else {
-      Fields<double> A = pr->F[pr->cur], B = pr->F[1 - pr->cur];
-      if (pr->order == PM_ORDER_JACOBI) {
-        CK(launch_sweep64(A, B, pr->codes, pr->list, pr->nlist, pr->g, pr->solver, pr->exact, 0,
-                          pr->st, pr->pf64[0]));
-      } else {
-        CK(launch_sweep64(A, B, pr->codes, pr->list, pr->nred, pr->g, pr->solver, pr->exact, 1,
-                          pr->st, pr->pf64[1]));
-        CK(launch_sweep64(A, B, pr->codes, pr->list + pr->nred, pr->nlist - pr->nred, pr->g,
-                          pr->solver, pr->exact, 2, pr->st, pr->pf64[2]));
-      }
+      pm_status s = sweeps64(pr, pr->F[pr->cur], pr->F[1 - pr->cur]);
+      if (s != PM_OK) return s;
     }
   }
   CK(cudaEventRecord(pr->ev1, pr->st));

@@ -80,7 +80,9 @@ struct pm_problem {
   int* list = nullptr;
   int nlist = 0;
   int nred = 0;             // red-black order: the list holds the red voxels first, then black
-  int pf64[3] = {1, 1, 1};  // per FP64 phase (Jacobi, red, black): launch form
+  int pf64[3] = {1, 1, 1};  // per FP64 phase (Jacobi, red, black): launch form alone
+  bool pf64_forced = false;
+  int share = 1;            // problems whose sweeps share the device, this one included
   double* f64_base[2] = {nullptr, nullptr};
   pm::Fields<double> F[2];
   float4* f32_base = nullptr;  // e0, e1, r (interleaved u, v, w, p)
@@ -136,6 +138,7 @@ struct pm_problem {
   // nothing else); each records the parities it ends with.
   struct BlockGraph {
     int n, cur, ecur, dc_pos, phase;  // phase: iteration % mixed_inner at the start
+    int share;
     int cur1, ecur1, dc_pos1;
     unsigned long long launches;
     cudaGraphExec_t exec;

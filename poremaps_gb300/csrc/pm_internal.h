@@ -52,6 +52,10 @@ struct Fields {
 // (cx, cy, cz) in 1..6 as 1 + (cx-1)*36 + (cy-1)*6 + (cz-1); 255 fluid halo.
 constexpr uint8_t kHaloFluid = 255;
 
+// What L2 holds of a working set that is swept again and again (129 MB, of which
+// the rest of a sweep's traffic takes a little).
+constexpr size_t kL2Bytes = 128u << 20;
+
 // Reduction partials: fixed grid so the summation order never changes.
 constexpr int kRedBlocks = 592;  // 4 x 148; fixed independent of the device
 constexpr int kRedThreads = 256;

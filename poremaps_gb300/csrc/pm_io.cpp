@@ -207,6 +207,7 @@ pm_status pm_solve_tensor(const pm_params* p, const uint8_t* geom, double K[9],
   auto run = [&](int a) {
     pm_problem* pr = nullptr;
     st[a] = problem_create(&ps[a], geom, a < 2 ? a : -1, &pr);
+    if (st[a] == PM_OK) pr->share = 3;
     if (st[a] == PM_OK) st[a] = pm_solve(pr, &r[a]);
     if (st[a] != PM_OK) err[a] = pm_last_error();
     pm_problem_destroy(pr);

@@ -309,7 +309,7 @@ bool flat_sweeps(const pm_server* s) {
 // them there.  Six samples of 5.8M voxels: 92 ms at 100 and 130 MB a group, 97
 // at 40, 96 in one group; 24 of 32..128: 64 ms at 130, 71 at 60, 97 at 20,
 // where groups are too small for the device, 65 in one.
-constexpr size_t kGroupBytes = 128u << 20;
+constexpr size_t kGroupBytes = kL2Bytes;
 
 void build_flat(pm_server* s) {
   size_t bytes = 0;

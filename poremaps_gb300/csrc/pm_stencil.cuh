@@ -434,7 +434,7 @@ __device__ __forceinline__ void update64(const Fields<double>& A, const Fields<d
   // 55.7 us; where it holds both (97x61x118, 112^3) as before; where it does not
   // hold one, without the hint (160^3 98 against 96 us, 224^3 217 against 203).
   // The same hint on a Jacobi sweep's reads of the plane below: 44.1 -> 45.1.
-  const bool one_fits = g.pl64 * g.NZ <= (128ll << 20) / 32;
+  const bool one_fits = g.pl64 * g.NZ <= (long long)kL2Bytes / 32;
   auto own = [&](const double* q) { return PHASE == 2 ? ld_last(q, one_fits) : ldA(q, LD); };
   o.u = own(U);
   o.v = own(V);

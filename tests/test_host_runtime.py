@@ -284,3 +284,31 @@ def test_failed_round_leaves_no_work_on_memory_that_is_kept(host, nth):
     assert L.fake_pending() == 0
     assert L.pm_server_cancel(s, t) == 0
     L.pm_server_destroy(s)
+
+
+# ------------------------------------------------------------------ problems beside each other
+@pytest.mark.parametrize("n,fluid,order,want", [
+    (128, 734000, pm.ORDER_REDBLACK, 3), (96, 500000, pm.ORDER_JACOBI, 3),  # beyond L2
+    (56, 105000, pm.ORDER_JACOBI, 2), (56, 105000, pm.ORDER_REDBLACK, 2),  # more than a wave
+    (24, 8300, pm.ORDER_JACOBI, 1), (48, 66000, pm.ORDER_REDBLACK, 1)])  # as alone
+def test_fp64_forms_of_problems_that_share_the_device(host, n, fluid, order, want):
+    """A group of three sweeps in the form that suits all three, whatever won
+    alone; the same problems by themselves sweep as before."""
+    L = host.L
+    L.pm_block_group_timed.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int] + \
+        [C.POINTER(C.c_double)] * 3
+    L.fake_set_cost(b"sweep64 form 1", 0.9)
+    hs = []
+    for _ in range(3):
+        st, h = host.create((n, n, n), fluid, order=order)
+        assert st == 0
+        hs.append(h)
+    host.trace()
+    for sweeps in (3, 20, 20):  # launched one by one, captured, replayed
+        three = (C.c_void_p * 3)(*hs)
+        assert L.pm_block_group_timed(three, 3, sweeps, 0, None, None, None) == 0
+        assert set(forms(host.trace())) <= {want}
+        assert L.pm_iterate(hs[0], sweeps) == 0
+        assert set(forms(host.trace())) <= {1}
+    for h in hs:
+        L.pm_problem_destroy(h)
