@@ -385,28 +385,36 @@ pm_status choose_fp64_shapes(pm_problem* pr) {
     for (int i = 0; i < 3; ++i) pr->pf64[i] = hit->second[i];
     return PM_OK;
   }
-  // whole iterations in turn between the two states, as a solve runs them; a
-  // second trial where they are short, and one voxel per thread only there (its
-  // gain is that it fills the device evenly)
-  constexpr float kLong = 1.0f;  // ms of a trial
-  auto set = [&](int form) { for (int& f : pr->pf64) f = form; };
+  // whole iterations in turn between the two states, as a solve runs them: every
+  // form once, then those within a tenth of the best again where iterations are
+  // short; one voxel per thread only where they are very short (it wins by the
+  // end of a wave if at all).  A 100^3 Jacobi problem of a new shape is set up in
+  // 1.63 ms so, 2.24 with nine iterations of every form.
+  constexpr float kShort = 0.25f, kVeryShort = 0.02f;  // ms an iteration
   float t[kForms64];
-  for (int form = kForms64 - 1; form >= 0; --form) {
-    t[form] = 1e30f;
-    if (form == kForm64One && t[kForm64Whole] >= kLong) break;
+  auto set = [&](int form) { for (int& f : pr->pf64) f = form; };
+  auto trial = [&](int form, int untimed, int timed) -> pm_status {
     set(form);
-    pm_status s = iterate64(pr);
-    for (int trial = 0; trial < 2 && s == PM_OK && !(trial && t[form] >= kLong); ++trial) {
-      CK(cudaEventRecord(pr->ev0, pr->st));
-      for (int r = 0; r < 4 && s == PM_OK; ++r) s = iterate64(pr);
-      CK(cudaEventRecord(pr->ev1, pr->st));
-      if (s == PM_OK) s = device_sync(pr, "FP64 sweep shape");
-      float ms = 0.f;
-      if (s == PM_OK) CK(cudaEventElapsedTime(&ms, pr->ev0, pr->ev1));
-      t[form] = std::min(t[form], ms);
-    }
+    pm_status s = PM_OK;
+    for (int r = 0; r < untimed && s == PM_OK; ++r) s = iterate64(pr);
     if (s != PM_OK) return s;
-  }
+    CK(cudaEventRecord(pr->ev0, pr->st));
+    for (int r = 0; r < timed && s == PM_OK; ++r) s = iterate64(pr);
+    CK(cudaEventRecord(pr->ev1, pr->st));
+    if (s == PM_OK) s = device_sync(pr, "FP64 sweep shape");
+    float ms = 0.f;
+    if (s == PM_OK) CK(cudaEventElapsedTime(&ms, pr->ev0, pr->ev1));
+    t[form] = std::min(t[form], ms / timed);
+    return s;
+  };
+  for (float& x : t) x = 1e30f;
+  pm_status s;
+  for (int form = kForms64 - 1; form >= 0; --form)
+    if (form != kForm64One || t[kForm64Whole] < kVeryShort)
+      if ((s = trial(form, 1, 2)) != PM_OK) return s;
+  const float near_best = 1.1f * *std::min_element(t, t + kForms64);
+  for (int form = kForms64 - 1; form >= 0; --form)
+    if (t[form] <= near_best && t[form] < kShort && (s = trial(form, 0, 4)) != PM_OK) return s;
   int best = kForm64Whole;
   for (int form = 0; form < kForm64Whole; ++form)
     if (t[form] < 0.99f * t[kForm64Whole] && t[form] < t[best]) best = form;

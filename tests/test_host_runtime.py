@@ -158,7 +158,7 @@ def test_fp64_form_is_timed(host, costs, want, scale):
         host.L.fake_set_cost(b"sweep64 form %d" % i, c * scale)
     st, h = host.create((40, 40, 40), 20000, order=pm.ORDER_JACOBI)
     assert st == 0
-    assert len(forms(host.trace())) <= (36 if scale < 0.1 else 15)
+    assert len(forms(host.trace())) <= (28 if scale < 0.1 else 9)
     assert host.L.pm_iterate(h, 2) == 0
     if scale == 1.0 and want == 0:
         want = 2
