@@ -14,9 +14,17 @@
 // an exchange copy of the fields, filled with kEmpty before the sweep: a tile
 // writes its outer columns' values there as it goes, and the next one polls
 // until they differ from kEmpty.  No flag and no fence is involved, since the
-// value itself is what arrives; and a tile's read of an old value comes before
-// the owner overwrites it, because the owner waits for a value computed from
-// it.  Every wait is bounded; when one runs out the sweep finishes without
+// value itself is what arrives.  A tile reads old values of the tiles above it
+// with plain loads, and their owners overwrite them with plain stores; no fence
+// orders the two.  What does is that the stored value is computed from a value
+// of the exchange which the reading tile computed from the old one: every old
+// value an update uses enters the velocity or pressure handed to the column it
+// came from, directly or through that column's neighbour.  A load that returned
+// the later store would depend on itself.  Programs may not produce such values
+// under PTX's memory model (its no-thin-air rule), and an SM does not issue a
+// store before the loads its data comes from have returned; but the plain
+// accesses are a race by the letter of that model, so this rests on the data
+// dependence and not on synchronisation.  Every wait is bounded; when one runs out the sweep finishes without
 // waiting and the host finds the error flag.
 //
 // What bounds it: GB300's FP64 pipe takes 64 clocks per instruction of a warp
