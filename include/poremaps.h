@@ -361,8 +361,10 @@ pm_status pm_debug_round_wait(unsigned extra, int polls);
  * and of the bulk-staged compact sweep (kernels 11 and 12) reports its first
  * pipeline wait as timed out without waiting: each CTA sets
  * the error flag, waits (bounded) for its copies in flight and returns, and
- * the sweep's caller gets PM_ERR_CUDA with the device still usable.  0 turns
- * it off.  Process-wide. */
+ * the sweep's caller gets PM_ERR_CUDA with the device still usable.  A launch of
+ * the reference order's sweep (captured blocks: those captured meanwhile) gives
+ * up each wait for a neighbour tile after one look, sets its error flag and
+ * finishes without waiting.  0 turns it off.  Process-wide. */
 pm_status pm_debug_tma_fail(int on);
 /* Problems made from now on sweep in the given launch form instead of the one
  * their timings pick, so a test can compare forms that lose on its machine:

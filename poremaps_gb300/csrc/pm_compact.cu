@@ -306,8 +306,10 @@ __global__ void k_pack_records(const unsigned* meta, const int4* sa, const int2*
 // Bound: the medium's values once they exceed L2 (64 bytes per voxel of e, r,
 // records and e2 against 76 with slots and metadata), the L1's gathers within
 // it.  Against kernels 10 / 9 (28 bytes of slots and metadata per voxel, plain
-// launches), per iteration of a solve: 48x48x64 pore 2.3 us (2.8), 128^3 pack
-// 7.8 (9.3), 157x93x211 9.5 (11.8), 256^3 38.9 (43.3), 512^3 309 (342).  The
+// launches), whole calls per iteration: 48x48x64 pore 2.8 to 3.0 us (3.3 to 3.5),
+// 128^3 pack 8.3 (9.8), 157x93x211 9.4 (11.9), 256^3 38.8 (43.3), 512^3 301 (342);
+// a sweep alone 7.7 us at 128^3, 34.8 at 256^3, 254 at 512^3 (64 bytes per voxel
+// at 0.92 and 1.01 of the measured copy rate).  The
 // streaming hint on r and the records is worth 8 % at 128^3 and 17 % when the
 // tensor's three problems share L2; bricks of the list instead of rows made no
 // difference at any size.
