@@ -85,18 +85,26 @@ bool pool_release() {
   return pool_give_back();
 }
 
+// An allocation, tried again when the kept blocks are given back; one that
+// failed is reported by its own status only, not by the next launch's
+// cudaGetLastError as well.
+template <typename Alloc>
+cudaError_t alloc_or_release(Alloc&& alloc, bool (*release)()) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (release()) e = alloc();
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 cudaError_t cuda_alloc(void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaErrorMemoryAllocation || !pool_release()) return e;
-  cudaGetLastError();
-  return cudaMalloc(p, bytes);
+  return alloc_or_release([&] { return cudaMalloc(p, bytes); }, pool_release);
 }
 
 cudaError_t cuda_alloc_async(void** p, size_t bytes, cudaStream_t st) {
-  cudaError_t e = cudaMallocAsync(p, bytes, st);
-  if (e != cudaErrorMemoryAllocation || !pool_release()) return e;
-  cudaGetLastError();
-  return cudaMallocAsync(p, bytes, st);
+  return alloc_or_release([&] { return cudaMallocAsync(p, bytes, st); }, pool_release);
 }
 
 template <typename T>
@@ -123,11 +131,7 @@ cudaError_t dev_alloc(T** ptr, size_t bytes) {
     g_pool_bytes -= bytes;
     g_pool.erase(g_pool.begin() + best);
   } else {
-    e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && pool_give_back()) {
-      cudaGetLastError();
-      e = cudaMalloc(&p, bytes);
-    }
+    e = alloc_or_release([&] { return cudaMalloc(&p, bytes); }, pool_give_back);
     if (e != cudaSuccess) return e;
   }
   g_pool_out[p] = {p, bytes, dev};

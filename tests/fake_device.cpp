@@ -42,7 +42,9 @@ std::map<void*, Block> g_blocks;
 std::set<Stream*> g_streams;
 std::map<std::string, double> g_cost;
 size_t g_total[2] = {64ull << 30, 64ull << 30}, g_used[2] = {0, 0};
+bool g_split = false;  // no block above half of a device's memory can be had
 int g_dev = 0, g_fluid = 0, g_fail_launch = 0;
+cudaError_t g_last = cudaSuccess;  // what cudaGetLastError returns, once
 bool g_capture = false;
 
 Stream* S(cudaStream_t st) { return (Stream*)st; }
@@ -59,6 +61,8 @@ enum { kPlain = 0, kOverlapped = 1 };
 cudaError_t launch(const char* name, cudaStream_t st, int how,
                    std::initializer_list<const void*> buffers) {
   if (g_fail_launch > 0 && --g_fail_launch == 0) return cudaErrorLaunchOutOfResources;
+  // the launchers report cudaGetLastError
+  if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
   note(name);
   for (const void* b : buffers)
     if (!b) note(std::string("null ") + name);
@@ -71,9 +75,9 @@ cudaError_t launch(const char* name, cudaStream_t st, int how,
 
 cudaError_t device_alloc(void** p, size_t n) {
   *p = nullptr;
-  if (g_used[g_dev] + n > g_total[g_dev]) {
+  if (g_used[g_dev] + n > g_total[g_dev] || (g_split && n > g_total[g_dev] / 2)) {
     note("out of memory");
-    return cudaErrorMemoryAllocation;
+    return g_last = cudaErrorMemoryAllocation;
   }
   void* m = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE,
                  -1, 0);
@@ -94,6 +98,7 @@ void fake_reset_trace() { g_trace.clear(); }
 void fake_set_fluid(int n) { g_fluid = n; }
 void fake_set_cost(const char* name, double ms) { g_cost[name] = ms; }
 void fake_set_memory(int dev, size_t bytes) { g_total[dev] = bytes; }
+void fake_split_memory(int on) { g_split = on != 0; }
 size_t fake_used(int dev) { return g_used[dev]; }
 void fake_fail_launch(int nth) { g_fail_launch = nth; }
 int fake_pending() {
@@ -136,7 +141,11 @@ cudaError_t cudaSetDevice(int d) {
   g_dev = d;
   return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = g_last;
+  g_last = cudaSuccess;
+  return e;
+}
 const char* cudaGetErrorString(cudaError_t e) {
   return e == cudaErrorMemoryAllocation ? "out of memory" : "error";
 }

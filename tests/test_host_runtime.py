@@ -236,6 +236,27 @@ def test_kept_blocks_are_bounded_and_given_back(host):
     L.pm_problem_destroy(h)
 
 
+def test_problem_after_one_that_did_not_fit(host):
+    """An allocation that failed is not reported by the launches of the next
+    problem."""
+    L = host.L
+    p = host.params((128, 128, 128), order=pm.ORDER_JACOBI)
+    need = C.c_size_t()
+    assert L.pm_problem_footprint(C.byref(p), C.byref(need)) == 0
+    # passes the check, which leaves out what alignment costs other problems
+    L.fake_set_memory(0, need.value + (1 << 20))
+    st, h = host.create((40, 40, 40), 1000, order=pm.ORDER_JACOBI)
+    assert st == 0
+    L.pm_problem_destroy(h)  # kept: counted as free, but not in one piece with the rest
+    L.fake_split_memory(1)
+    st, _ = host.create((128, 128, 128), 1000, order=pm.ORDER_JACOBI)
+    assert st == pm.PM_ERR_NOMEM and b"out of memory" in L.pm_last_error()
+    L.fake_split_memory(0)
+    st, h = host.create((40, 40, 40), 1000, order=pm.ORDER_JACOBI)
+    assert st == 0, L.pm_last_error()
+    L.pm_problem_destroy(h)
+
+
 @pytest.mark.parametrize("left", [0, 1 << 12])
 def test_any_allocation_gets_what_is_kept(host, left):
     """Not only a problem's own buffers: where the server's tables do not fit
